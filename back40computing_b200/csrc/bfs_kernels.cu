@@ -15,7 +15,8 @@
 //   * lists >= cta_th are cut, when their vertex is discovered, into chunks of
 //     16 * THREADS edges for the NEXT level; there every CTA of the grid takes
 //     chunks in turn and streams each with all its threads (CTA-based gather,
-//     spread over the grid so a hub never serialises a level);
+//     spread over the grid so a hub never serialises a level; a level of few
+//     chunks goes out in smaller slices);
 //   * lists >= warp_th are streamed by one warp (warp-based gather);
 //   * shorter lists are packed by a warp prefix sum into a per-warp shared
 //     memory window of gather offsets that the warp reads together
@@ -299,10 +300,9 @@ __device__ __forceinline__ unsigned place_tier(int4 *table, unsigned *count, int
 // with their lanes.  Returns the bits of the lists placed in a chunk table.
 // Called by all lanes together.
 // c: the counters the chunk counts go to (p.ctr, or a narrow launch's copy).
-template <int THREADS>
+template <int CH>
 __device__ __forceinline__ unsigned place4(const BfsParams &p, int q_next, unsigned has, const int (&st)[4],
                                            const int (&ln)[4], const int (&pr)[4], Counters *c) {
-    constexpr int CH = chunk_edges<THREADS>();
     unsigned cta = 0, wrp = 0;
     int ncta = 0, nw = 0, nc[4];
 #pragma unroll
@@ -327,30 +327,15 @@ __device__ __forceinline__ unsigned place4(const BfsParams &p, int q_next, unsig
     placed |= place_tier<WARP_CHUNK>(p.wchunks[nq], &c->wch[q_next & 3], p.wchunk_cap, wrp, nw, nc, st, ln, pr);
     return placed;
 }
-template <int THREADS>
+template <int CH>
 __device__ __forceinline__ unsigned place4(const BfsParams &p, int q_next, unsigned has, const int (&st)[4],
                                            const int (&ln)[4], const int (&pr)[4]) {
-    return place4<THREADS>(p, q_next, has, st, ln, pr, p.ctr);
+    return place4<CH>(p, q_next, has, st, ln, pr, p.ctr);
 }
 
 // ---------------------------------------------------------------------------------------
 // Gather strategies
 // ---------------------------------------------------------------------------------------
-
-// Grid-wide chunk phase: CTA b streams chunks b, b + G, b + 2G, ... of table.
-template <int THREADS, class Sink>
-__device__ __forceinline__ void gather_chunks(const BfsParams &p, const int4 *table, unsigned n, const Sink &sink,
-                                              uint64_t pol) {
-    if (n > (unsigned)p.chunk_cap) n = p.chunk_cap;
-    const unsigned G = gridDim.x;
-    unsigned k = blockIdx.x;
-    int4 cur = k < n ? __ldcg(table + k) : make_int4(0, 0, 0, 0);
-    for (; k < n; k += G) {
-        int4 nxt = (k + G < n) ? __ldcg(table + k + G) : make_int4(0, 0, 0, 0);
-        if (cur.y > 0) gather_list<THREADS>(p.col, p.vec_end, cur.x, cur.y, cur.z, 0u, threadIdx.x, sink, pol);
-        cur = nxt;
-    }
-}
 
 // Warp w of the grid is warp w / gridDim.x of CTA w % gridDim.x: consecutive
 // work items (tiles, steps, runs) go to different CTAs, and so to different
@@ -359,47 +344,61 @@ __device__ __forceinline__ void gather_chunks(const BfsParams &p, const int4 *ta
 __device__ __forceinline__ int global_warp() { return int((threadIdx.x >> 5) * gridDim.x + blockIdx.x); }
 __device__ __forceinline__ int grid_warps() { return int(gridDim.x * (blockDim.x >> 5)); }
 
-// Warp chunk phase: warp w of the grid streams warp chunks w, w + W, ...
-template <class Sink>
-__device__ __forceinline__ void gather_wchunks(const BfsParams &p, const int4 *table, unsigned n, const Sink &sink,
-                                               uint64_t pol) {
-    if (n > (unsigned)p.wchunk_cap) n = p.wchunk_cap;
-    const unsigned W = grid_warps();
-    unsigned k = global_warp();
-    int4 cur = k < n ? __ldcg(table + k) : make_int4(0, 0, 0, 0);
-    for (; k < n; k += W) {
-        int4 nxt = (k + W < n) ? __ldcg(table + k + W) : make_int4(0, 0, 0, 0);
+// Whole chunks: CTA b streams CTA chunks b, b + G, ..., then warp w of the
+// grid warp chunks w, w + W, ...
+template <int THREADS, class Sink>
+__device__ __forceinline__ void gather_whole_chunks(const BfsParams &p, const int4 *ctable, unsigned nch,
+                                                    const int4 *wtable, unsigned nw, const Sink &sink,
+                                                    uint64_t pol) {
+    const unsigned G = gridDim.x, W = grid_warps();
+    unsigned k = blockIdx.x;
+    int4 cur = k < nch ? __ldcg(ctable + k) : make_int4(0, 0, 0, 0);
+    for (; k < nch; k += G) {
+        const int4 nxt = k + G < nch ? __ldcg(ctable + k + G) : make_int4(0, 0, 0, 0);
+        if (cur.y > 0) gather_list<THREADS>(p.col, p.vec_end, cur.x, cur.y, cur.z, 0u, threadIdx.x, sink, pol);
+        cur = nxt;
+    }
+    k = global_warp();
+    cur = k < nw ? __ldcg(wtable + k) : make_int4(0, 0, 0, 0);
+    for (; k < nw; k += W) {
+        const int4 nxt = k + W < nw ? __ldcg(wtable + k + W) : make_int4(0, 0, 0, 0);
         if (cur.y > 0) gather_list<32>(p.col, p.vec_end, cur.x, cur.y, cur.z, 0u, lane_id(), sink, pol);
         cur = nxt;
     }
 }
 
-// Both chunk tables of a phase.  When their slices of 128 edges (one 16-byte
-// load per lane) number no more than the grid's warps, every warp takes one
-// slice: a small level then finishes in one pass instead of the 4 passes a
-// CTA or warp needs for a whole chunk.  Otherwise CTAs stream CTA chunks and
-// warps stream warp chunks.
-template <int THREADS, class Sink>
+// Both chunk tables of a phase.  While the CTA chunks number fewer than the
+// CTAs and the warp chunks fewer than the warps, whole chunks would leave
+// part of the grid idle (82 CTA chunks kept 82 of 296 CTAs busy): the tables
+// are cut into slices of 128 edges, one 16-byte load per lane, that go to the
+// grid's warps in turn.  Slices past a chunk's end are empty and cost one
+// descriptor read.  Larger tables, where they would be most of the work, go
+// out as whole chunks.  So do those of predecessor searches, unless every warp
+// has at most one slice: which of a vertex's possible parents is recorded
+// depends on the order in which the lists are streamed, and callers that
+// compare parent arrays see it change (the slices changed 1.4% of the parents
+// on R-MAT scale 18, against 0.6% from run to run).
+template <int THREADS, bool MP, class Sink>
 __device__ __forceinline__ void gather_chunk_tables(const BfsParams &p, const int4 *ctable, unsigned nch,
                                                     const int4 *wtable, unsigned nw, const Sink &sink,
                                                     uint64_t pol) {
     constexpr unsigned SLICE = 128;
-    constexpr unsigned CS = chunk_edges<THREADS>() / SLICE, WS = WARP_CHUNK / SLICE;
+    constexpr unsigned CS = chunk_edges<THREADS>() / SLICE, WS = WARP_CHUNK / SLICE;  // powers of two
     if (nch > (unsigned)p.chunk_cap) nch = p.chunk_cap;
     if (nw > (unsigned)p.wchunk_cap) nw = p.wchunk_cap;
+    const unsigned W = grid_warps();
     const unsigned long long slices = (unsigned long long)nch * CS + (unsigned long long)nw * WS;
-    if (slices > (unsigned long long)grid_warps()) {
-        gather_chunks<THREADS>(p, ctable, nch, sink, pol);
-        gather_wchunks(p, wtable, nw, sink, pol);
+    if (MP ? slices > (unsigned long long)W : nch >= gridDim.x || nw >= W) {
+        gather_whole_chunks<THREADS>(p, ctable, nch, wtable, nw, sink, pol);
         return;
     }
-    const unsigned w = global_warp();
-    if (w >= slices) return;
-    const int4 ch = w < nch * CS ? __ldcg(ctable + w / CS) : __ldcg(wtable + (w - nch * CS) / WS);
-    const unsigned k = w < nch * CS ? w % CS : (w - nch * CS) % WS;
-    const int a0 = (ch.x & ~3) + int(k * SLICE);
-    const int s0 = max(a0, ch.x), e0 = min(a0 + int(SLICE), ch.x + ch.y);
-    if (e0 > s0) gather_list<32>(p.col, p.vec_end, s0, e0 - s0, ch.z, 0u, lane_id(), sink, pol);
+    const unsigned nc = nch * CS, n = nc + nw * WS;  // below W * (CS + WS)
+    for (unsigned k = global_warp(); k < n; k += W) {
+        const int4 ch = __ldcg(k < nc ? ctable + k / CS : wtable + (k - nc) / WS);
+        const int a = (ch.x & ~3) + int((k < nc ? k % CS : (k - nc) % WS) * SLICE);
+        const int s0 = max(a, ch.x), e0 = min(a + int(SLICE), ch.x + ch.y);
+        if (e0 > s0) gather_list<32>(p.col, p.vec_end, s0, e0 - s0, ch.z, 0u, lane_id(), sink, pol);
+    }
 }
 
 // ---- window gathers of up to 4 lists per lane ------------------------------------------
@@ -533,23 +532,34 @@ __device__ __forceinline__ void gather_windows4(const BfsParams &p, WarpSmem<MP>
     }
 }
 
-// Frontier vertices per lane of a warp tile: 4 (tiles of WINDOW vertices, row
-// ranges and lists of four vertices per lane in flight together) once a level
-// has at least two such tiles per warp of the grid, else 1 (tiles of 32), so
-// that a small level still gives every warp of the grid a tile.
-__device__ __forceinline__ unsigned vertices_per_lane(unsigned L) {
-    return (unsigned long long)L >= 2ull * WINDOW * unsigned(grid_warps()) ? 4u : 1u;
+// Queue entries per warp tile of a level of L entries, a power of two: WINDOW
+// (4 per lane, their row ranges and lists in flight together) once a level
+// has two such tiles per warp of the grid; below, one tile per warp, of at
+// most `small` entries, so that the lists of a tile's vertices, which its warp
+// streams window after window in a chain, spread over the grid's idle warps:
+// on a random graph of mean degree 16 a level of 355 edges took 20.9 us in 3
+// tiles of 128 and takes 7.2 us in 45 of 8.  Not below p.tile_min entries,
+// about one window of edges at the graph's mean degree, because each tile
+// makes a queue reservation of its own (lattices, short lists).  Predecessor
+// searches keep tiles of `small` for the order's sake (gather_chunk_tables).
+template <bool MP>
+__device__ __forceinline__ unsigned tile_width(const BfsParams &p, unsigned L, unsigned small) {
+    const unsigned W = unsigned(grid_warps());
+    if ((unsigned long long)L >= 2ull * WINDOW * W) return unsigned(WINDOW);
+    if (MP) return small;
+    const unsigned want = max((L + W - 1u) / W, p.tile_min);
+    return min(small, 1u << (32 - __clz(int(want) - 1)));
 }
 
-// Loads the frontier vertices of warp tile t (per vertices per lane, tile
-// size 32 * per) from q_in; bit j of the result marks v[j].
-__device__ __forceinline__ unsigned load_tile(const int *q_in, unsigned L, unsigned t, unsigned per, int (&v)[4]) {
+// Loads the frontier vertices of warp tile t (tiles of tw entries) from q_in;
+// bit j of the result marks v[j].
+__device__ __forceinline__ unsigned load_tile(const int *q_in, unsigned L, unsigned t, unsigned tw, int (&v)[4]) {
     unsigned sel = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const unsigned idx = t * 32u * per + unsigned(j) * 32u + lane_id();
+        const unsigned at = unsigned(j) * 32u + lane_id(), idx = t * tw + at;
         v[j] = -1;
-        if (unsigned(j) < per && idx < L) {
+        if (at < tw && idx < L) {
             v[j] = ld_cg(q_in + idx);
             sel |= 1u << j;
         }
@@ -804,7 +814,7 @@ struct DiscoverSink {
             if ((disc >> j) & 1u) p.labels[u[j]] = MP ? pred[j] : label;
         if (p.do_alpha)
             count_discovered(sm.w[threadIdx.x >> 5], __popc(disc), (long long)ln[0] + ln[1] + ln[2] + ln[3]);
-        const unsigned enq = disc & ~place4<THREADS>(p, label, disc, st, ln, u);
+        const unsigned enq = disc & ~place4<chunk_edges<THREADS>()>(p, label, disc, st, ln, u);
         stage4(sm.w[threadIdx.x >> 5], enq, u, q_out, qlen_out, p.qcap, &p.ctr->error);
     }
     __device__ __forceinline__ void drain() const {
@@ -880,7 +890,7 @@ struct ContractExpandSink {
             if ((surv >> j) & 1u) p.labels[u[j]] = MP ? pred[j] : it;
         WarpSmem<MP> &ws = sm.w[threadIdx.x >> 5];
         if (p.count_raw) count_raw(&ws.raw_n, has, ln);
-        const unsigned placed = place4<THREADS>(p, q + 1, has, st, ln, u);
+        const unsigned placed = place4<chunk_edges<THREADS>()>(p, q + 1, has, st, ln, u);
         const unsigned rest = has & ~placed;
         const int nq = (q + 1) & 1;
         // Stage the short lists; gather when the stage would overflow.
@@ -956,7 +966,7 @@ struct ContractSink {
 // ---------------------------------------------------------------------------------------
 
 // Expand-contract level it: vertex frontier -> discovered vertices labelled it+1.
-// Warp tiles of frontier vertices (vertices_per_lane): their row ranges are
+// Warp tiles of frontier vertices (tile_width): their row ranges are
 // loaded together and their lists streamed by one window gather into the
 // discovery sink.
 template <int THREADS, bool MP>
@@ -967,18 +977,18 @@ __device__ void ec_level(const BfsParams &p, int it, unsigned L, unsigned nch, u
     // a vertex queue's lists are shorter than warp_th; count 16 entries each
     DiscoverSink<THREADS, MP> sink{p, sm, p.queue[nq], &c->qlen[(it + 1) & 3], it + 1,
                                    probe_level(phase_work<THREADS>(L, 16u, nch, nwch))};
-    gather_chunk_tables<THREADS>(p, p.chunks[it & 1], nch, p.wchunks[it & 1], nwch, sink, pol);
+    gather_chunk_tables<THREADS, MP>(p, p.chunks[it & 1], nch, p.wchunks[it & 1], nwch, sink, pol);
     WarpSmem<MP> &ws = sm.w[threadIdx.x >> 5];
     const int *q_in = p.queue[it & 1];
-    const unsigned per = vertices_per_lane(L);
-    const unsigned ntiles = (L + 32u * per - 1) / (32u * per);
+    const unsigned tw = tile_width<MP>(p, L, 32u);
+    const unsigned ntiles = (L + tw - 1u) / tw;
     const unsigned grab = tile_grab(ntiles);
     const unsigned nruns = (ntiles + grab - 1) / grab;
     for (unsigned r = global_warp(); r < nruns; r = next_run(nruns, &c->steal[it & 3])) {
         const unsigned t0 = r * grab;
         for (unsigned t = t0; t < t0 + grab && t < ntiles; t++) {
             int v[4], st[4], ln[4];
-            const unsigned sel = load_tile(q_in, L, t, per, v);
+            const unsigned sel = load_tile(q_in, L, t, tw, v);
             const unsigned has = row_ranges4(p, sel, v, st, ln);
             gather_windows4<MP>(p, ws, has, st, ln, v, sink, pol);
         }
@@ -1215,7 +1225,7 @@ __device__ __forceinline__ void bu_step(const BfsParams &p, int it, unsigned w0,
         }
     }
     count_discovered(ws, nfound, dfound);
-    const unsigned placed = place4<THREADS>(p, it + 1, found, st, ln, v);
+    const unsigned placed = place4<chunk_edges<THREADS>()>(p, it + 1, found, st, ln, v);
     stage4(ws, found & ~placed, v, q_out, qlen_out, p.qcap, &c->error);
 }
 
@@ -1328,21 +1338,22 @@ __device__ void bu_level(const BfsParams &p, int it, Smem<THREADS, MP> &sm, unsi
     flush_discovered(p, ws, it + 1);
 }
 
-// Edge-frontier phase input: warp tiles of 128 elements (4 per lane,
-// coalesced), statically interleaved over the grid's warps.
+// Edge-frontier phase input: warp tiles of tw elements (tile_width; coalesced),
+// statically interleaved over the grid's warps.
 template <bool MP, class Sink>
-__device__ __forceinline__ void edge_tiles(const int *q_in, const int *pq_in, unsigned L, const Sink &sink) {
-    const unsigned ntiles = (L + WINDOW - 1) / WINDOW;
+__device__ __forceinline__ void edge_tiles(const int *q_in, const int *pq_in, unsigned L, unsigned tw,
+                                           const Sink &sink) {
+    const unsigned ntiles = (L + tw - 1u) / tw;
     const unsigned W = grid_warps();
     for (unsigned t = global_warp(); t < ntiles; t += W) {
         unsigned valid = 0;
         int u[4], pr[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const unsigned idx = t * WINDOW + j * 32 + lane_id();
+            const unsigned at = unsigned(j) * 32u + lane_id(), idx = t * tw + at;
             u[j] = -1;
             pr[j] = 0;
-            if (idx < L) {
+            if (at < tw && idx < L) {
                 valid |= 1u << j;
                 u[j] = ld_cg(q_in + idx);
                 if (MP) pr[j] = ld_cg(pq_in + idx);
@@ -1358,8 +1369,8 @@ template <int THREADS, bool MP>
 __device__ void ce_level(const BfsParams &p, int it, int q, unsigned L, unsigned nch, unsigned nwch,
                          Smem<THREADS, MP> &sm, uint64_t pol) {
     ContractExpandSink<THREADS, MP> sink{p, sm, it, q, pol, probe_level(phase_work<THREADS>(L, 1u, nch, nwch))};
-    gather_chunk_tables<THREADS>(p, p.chunks[q & 1], nch, p.wchunks[q & 1], nwch, sink, pol);
-    edge_tiles<MP>(p.queue[q & 1], p.pred_queue[q & 1], L, sink);
+    gather_chunk_tables<THREADS, MP>(p, p.chunks[q & 1], nch, p.wchunks[q & 1], nwch, sink, pol);
+    edge_tiles<MP>(p.queue[q & 1], p.pred_queue[q & 1], L, tile_width<MP>(p, L, unsigned(WINDOW)), sink);
     sink.drain();
 }
 
@@ -1369,13 +1380,13 @@ __device__ void tp_contract(const BfsParams &p, int it, int qi, unsigned L, unsi
                             Smem<THREADS, MP> &sm, uint64_t pol) {
     ContractSink<THREADS, MP> sink{p, sm, p.queue[(qi + 1) & 1], &p.ctr->qlen[(qi + 1) & 3], it,
                                    probe_level(phase_work<THREADS>(L, 1u, nch, nwch))};
-    gather_chunk_tables<THREADS>(p, p.chunks[qi & 1], nch, p.wchunks[qi & 1], nwch, sink, pol);
-    edge_tiles<MP>(p.queue[qi & 1], p.pred_queue[qi & 1], L, sink);
+    gather_chunk_tables<THREADS, MP>(p, p.chunks[qi & 1], nch, p.wchunks[qi & 1], nwch, sink, pol);
+    edge_tiles<MP>(p.queue[qi & 1], p.pred_queue[qi & 1], L, unsigned(WINDOW), sink);
     sink.drain();
 }
 
 // Two-phase expand, phase qi = 2 * it + 1 (two_phase/expand_atomic/cta.cuh:606-719):
-// warp tiles of frontier vertices (vertices_per_lane); long lists become
+// warp tiles of frontier vertices (tile_width); long lists become
 // chunks of the next phase, the others are streamed by one window gather per
 // tile through the gather-time cull into the next edge frontier.
 template <int THREADS, bool MP>
@@ -1385,18 +1396,18 @@ __device__ void tp_expand(const BfsParams &p, int qi, unsigned L, bool cull, Sme
     WarpSmem<MP> &ws = sm.w[threadIdx.x >> 5];
     const FilterSink<THREADS, MP> out{p, sm, p.queue[nq], p.pred_queue[nq], &c->qlen[(qi + 1) & 3]};
     const int *q_in = p.queue[qi & 1];
-    const unsigned per = vertices_per_lane(L);
-    const unsigned ntiles = (L + 32u * per - 1) / (32u * per);
+    const unsigned tw = tile_width<MP>(p, L, 32u);
+    const unsigned ntiles = (L + tw - 1u) / tw;
     const unsigned grab = tile_grab(ntiles);
     const unsigned nruns = (ntiles + grab - 1) / grab;
     for (unsigned r = global_warp(); r < nruns; r = next_run(nruns, &c->steal[qi & 3])) {
         const unsigned t0 = r * grab;
         for (unsigned t = t0; t < t0 + grab && t < ntiles; t++) {
             int v[4], st[4], ln[4];
-            const unsigned sel = load_tile(q_in, L, t, per, v);
+            const unsigned sel = load_tile(q_in, L, t, tw, v);
             const unsigned has = row_ranges4(p, sel, v, st, ln);
             if (cull || p.count_raw) count_raw(&ws.raw_n, has, ln);
-            const unsigned placed = place4<THREADS>(p, qi + 1, has, st, ln, v);
+            const unsigned placed = place4<chunk_edges<THREADS>()>(p, qi + 1, has, st, ln, v);
             if (cull)
                 gather_windows4<MP>(p, ws, has & ~placed, st, ln, v, out, pol);
             else
@@ -1688,7 +1699,7 @@ __device__ void ec_narrow_level(const BfsParams &p, Counters *c, int it, unsigne
                 dm += unsigned(ln[j]);
             }
             dn += unsigned(__popc(disc));
-            const unsigned enq = disc & ~place4<THREADS>(p, label, disc, st, ln, v, c);
+            const unsigned enq = disc & ~place4<chunk_edges<THREADS>()>(p, label, disc, st, ln, v, c);
             unsigned total = 0, pre[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -1821,7 +1832,7 @@ __device__ void ce_narrow_level(const BfsParams &p, Counters *c, int it, unsigne
         const int len = claimed ? r1 - r0 : 0;
         if (p.count_raw) raw += unsigned(len);
         const int st4[4] = {r0, 0, 0, 0}, ln4[4] = {len, 0, 0, 0}, own4[4] = {u, 0, 0, 0};
-        const unsigned placed = place4<THREADS>(p, it + 1, len > 0 ? 1u : 0u, st4, ln4, own4, c);
+        const unsigned placed = place4<chunk_edges<THREADS>()>(p, it + 1, len > 0 ? 1u : 0u, st4, ln4, own4, c);
         const int n = placed ? 0 : len;
         const int incl = warp_inclusive_scan(n);
         const unsigned total = (unsigned)__shfl_sync(FULL, incl, 31);
@@ -1894,7 +1905,7 @@ __device__ void ce_flat_level(const BfsParams &p, int it, int q, unsigned L, Sme
         const int len = claimed ? r1v - r0v : 0;
         if (p.count_raw) raw += unsigned(len);
         const int st4[4] = {r0v, 0, 0, 0}, ln4[4] = {len, 0, 0, 0}, own4[4] = {u, 0, 0, 0};
-        const unsigned placed = place4<THREADS>(p, q + 1, len > 0 ? 1u : 0u, st4, ln4, own4);
+        const unsigned placed = place4<chunk_edges<THREADS>()>(p, q + 1, len > 0 ? 1u : 0u, st4, ln4, own4);
         const int n = placed ? 0 : len;
         int first[4];
 #pragma unroll
@@ -2207,7 +2218,7 @@ __device__ void tp_narrow_expand(const BfsParams &p, Counters *c, int qi, unsign
         const int len = ok ? __ldg(p.row_offsets + u + 1) - r0 : 0;
         if (p.count_raw) raw += unsigned(len);
         const int st4[4] = {r0, 0, 0, 0}, ln4[4] = {len, 0, 0, 0}, own4[4] = {u, 0, 0, 0};
-        const unsigned placed = place4<THREADS>(p, qi + 1, len > 0 ? 1u : 0u, st4, ln4, own4, c);
+        const unsigned placed = place4<chunk_edges<THREADS>()>(p, qi + 1, len > 0 ? 1u : 0u, st4, ln4, own4, c);
         const int n = placed ? 0 : len;
         const int incl = warp_inclusive_scan(n);
         const unsigned total = (unsigned)__shfl_sync(FULL, incl, 31);

@@ -89,7 +89,16 @@ struct BfsParams {
     // Full-grid levels of at most flat_max queued edges without chunked lists
     // run contract-expand's latency-first body (ce_flat_level); 0: never.
     unsigned flat_max;
+    // Smallest warp tile of a queued frontier (tile_width): min_tile().
+    unsigned tile_min;
 };
+
+// Queue entries whose lists are about one 128-entry window of edges at the
+// graph's mean degree.
+inline unsigned min_tile(long long nodes, long long edges) {
+    const long long t = edges > 0 ? 128 * nodes / edges : 128;
+    return unsigned(t < 4 ? 4 : t > 128 ? 128 : t);
+}
 
 // Padding of the device arrays a staged bottom-up step copies in whole
 // 16-byte units past their ends.
