@@ -72,6 +72,7 @@ struct b40c_problem {
     bool reset_once = false;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
+    long long max_degree = 0;              // longest list of the uploaded graph
     int symmetric = -1;                    // -1 unknown, 0 no, 1 yes (checked on first use)
     unsigned long long *d_sym = nullptr;   // 4 hash sums of the symmetry check
     unsigned *d_mask_snap = nullptr;       // predecessor-label bottom-up levels: visited-mask copy
@@ -98,7 +99,7 @@ struct b40c_enactor {
     int threads = 256;
     int warp_th = 64, cta_th = 1024;
     unsigned cull_flags = CULL_HISTORY;
-    unsigned do_alpha = 0, do_beta = 0;  // direction-optimizing expand-contract (0: top-down only)
+    unsigned do_alpha = 0, do_beta = 0;  // direction switch (0: top-down only)
     unsigned long long wait_ns = 5000000000ull;
     int l2_persist = 0;  // b40c_enactor_set_l2_persistence
     bool stage_bu = false;  // b40c_enactor_set_bottom_up_staging
@@ -248,8 +249,9 @@ int ensure_heavy_known(b40c_problem *p) {
 int device_check_csr(b40c_problem *p, const int *h_row, const int *h_col) {
     cudaStream_t s = problem_stream(p);
     if (!p->d_sym) CUDA_TRY(cudaMalloc(&p->d_sym, 4 * sizeof(unsigned long long)), "cudaMalloc check buffer");
-    unsigned long long h[2];
-    CUDA_TRY(cudaMemsetAsync(p->d_sym, 0xff, sizeof(h), s), "CSR check clear");
+    unsigned long long h[3];
+    CUDA_TRY(cudaMemsetAsync(p->d_sym, 0xff, 2 * sizeof(h[0]), s), "CSR check clear");
+    CUDA_TRY(cudaMemsetAsync(p->d_sym + 2, 0, sizeof(h[0]), s), "CSR check clear");
     CUDA_TRY(launch_csr_check(p->d_row_offsets, p->d_col, int(p->nodes), p->edges, p->d_sym, s), "CSR check launch");
     CUDA_TRY(cudaMemcpyAsync(h, p->d_sym, sizeof(h), cudaMemcpyDeviceToHost, s), "CSR check copy");
     CUDA_TRY(cudaStreamSynchronize(s), "CSR check");
@@ -258,6 +260,7 @@ int device_check_csr(b40c_problem *p, const int *h_row, const int *h_col) {
     if (h[1] != ~0ull)
         return set_error(B40C_ERR_INVALID_VALUE, "CSR column index %d at edge %lld outside [0, %lld)",
                          h_col[h[1]], (long long)h[1], (long long)p->nodes);
+    p->max_degree = (long long)h[2];
     return B40C_SUCCESS;
 }
 
@@ -441,11 +444,17 @@ int enqueue_search(b40c_enactor *e, b40c_problem *p, int src, int max_grid_size,
     // The hybrid switches between its two bodies inside one persistent launch;
     // like the reference's EnactorHybrid it has a single way to run a search.
     if (variant == B40C_VARIANT_DEFAULT || e->strategy == B40C_HYBRID) variant = B40C_VARIANT_FUSED;
-    // Bottom-up levels: fused expand-contract on a symmetric graph held on the
-    // device (their scattered column reads would cross PCIe one entry at a time
-    // from a stream_from_host graph); with predecessor labels they probe a copy
-    // of the visited mask.
-    if (e->strategy == B40C_EXPAND_CONTRACT && variant == B40C_VARIANT_FUSED && e->do_alpha && !p->mapped) {
+    // Bottom-up levels: fused searches on a symmetric graph held on the device
+    // (their scattered column reads would cross PCIe one entry at a time from a
+    // stream_from_host graph).  With predecessor labels they probe a copy of
+    // the visited mask, and only expand-contract runs them: the other
+    // strategies' predecessors stay the ones their top-down levels record.
+    // On low-degree graphs the other strategies stay top-down too (counting
+    // their edge frontiers and sweeping the last levels took the 256^3 lattice
+    // from 4.5 to 8.0 ms).
+    if (variant == B40C_VARIANT_FUSED && e->do_alpha && !p->mapped &&
+        (e->strategy == B40C_EXPAND_CONTRACT ||
+         (edge_switch(e->threads, p->mark_pred) && p->max_degree > LOW_DEGREE))) {
         if ((rc = ensure_symmetry_known(p))) return rc;
         if (p->symmetric == 1) {
             if (p->mark_pred && p->mask_snap_cap < p->mask_bytes) {
@@ -458,10 +467,13 @@ int enqueue_search(b40c_enactor *e, b40c_problem *p, int src, int max_grid_size,
             if ((rc = ensure_heavy_known(p))) return rc;
             bp.mask_snap = p->d_mask_snap;
             bp.heavy = p->d_heavy;
-            bp.stage_bu = e->stage_bu ? 1 : 0;  // the problem's row offsets, mask and keys carry the padding
-            kc.stage_bu = e->stage_bu;           // and the launch carries the stage buffers
+            // the problem's row offsets, mask and keys carry the padding, and
+            // the expand-contract launch the stage buffers
+            kc.stage_bu = e->stage_bu && e->strategy == B40C_EXPAND_CONTRACT;
+            bp.stage_bu = kc.stage_bu ? 1 : 0;
             bp.do_alpha = e->do_alpha;
             bp.do_beta = e->do_beta;
+            if (e->strategy != B40C_EXPAND_CONTRACT) bp.count_raw = 1;  // the edge frontiers decide the direction
         }
     }
     if (bp.levels)
@@ -1004,20 +1016,15 @@ extern "C" int b40c_enactor_create(int strategy, int instrument, int debug, b40c
     b40c_enactor *e = new (std::nothrow) b40c_enactor();
     if (!e) return set_error(B40C_ERR_MEMORY_ALLOCATION, "enactor allocation");
     e->strategy = strategy;
-    // Measured defaults: expand-contract and contract-expand run 512-thread
-    // CTAs (best for both on R-MAT scale 22 and on the lattices); two-phase
-    // and the hybrid run 256-thread CTAs (best on R-MAT scale 22).
+    // Measured defaults: 512-thread CTAs (best on R-MAT scale 22 and on the
+    // lattices; the edge-frontier strategies' direction switch needs them).
     // Expand-contract gathers lists of 128+ edges with warps, the others lists
-    // of 64+, and expand-contract switches direction with the published
-    // alpha = 14, beta = 24 (Beamer, Asanovic and Patterson, SC 2012).
-    if (strategy == B40C_EXPAND_CONTRACT) {
-        e->threads = 512;
-        e->warp_th = 128;
-        e->do_alpha = 14;
-        e->do_beta = 24;
-    } else if (strategy == B40C_CONTRACT_EXPAND) {
-        e->threads = 512;
-    }
+    // of 64+, and every strategy switches direction with the published alpha =
+    // 14, beta = 24 (Beamer, Asanovic and Patterson, SC 2012).
+    e->threads = 512;
+    e->do_alpha = 14;
+    e->do_beta = 24;
+    if (strategy == B40C_EXPAND_CONTRACT) e->warp_th = 128;
     e->instrument = instrument != 0;
     e->debug = debug != 0;
     cudaError_t ce = cudaGetDevice(&e->device);

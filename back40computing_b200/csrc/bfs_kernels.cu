@@ -344,24 +344,31 @@ __device__ __forceinline__ unsigned place4(const BfsParams &p, int q_next, unsig
 __device__ __forceinline__ int global_warp() { return int((threadIdx.x >> 5) * gridDim.x + blockIdx.x); }
 __device__ __forceinline__ int grid_warps() { return int(gridDim.x * (blockDim.x >> 5)); }
 
-// Whole chunks: CTA b streams CTA chunks b, b + G, ..., then warp w of the
-// grid warp chunks w, w + W, ...
+// Grid-wide chunk phase: CTA b streams chunks b, b + G, b + 2G, ... of table.
 template <int THREADS, class Sink>
-__device__ __forceinline__ void gather_whole_chunks(const BfsParams &p, const int4 *ctable, unsigned nch,
-                                                    const int4 *wtable, unsigned nw, const Sink &sink,
-                                                    uint64_t pol) {
-    const unsigned G = gridDim.x, W = grid_warps();
+__device__ __forceinline__ void gather_chunks(const BfsParams &p, const int4 *table, unsigned n, const Sink &sink,
+                                              uint64_t pol) {
+    if (n > (unsigned)p.chunk_cap) n = p.chunk_cap;
+    const unsigned G = gridDim.x;
     unsigned k = blockIdx.x;
-    int4 cur = k < nch ? __ldcg(ctable + k) : make_int4(0, 0, 0, 0);
-    for (; k < nch; k += G) {
-        const int4 nxt = k + G < nch ? __ldcg(ctable + k + G) : make_int4(0, 0, 0, 0);
+    int4 cur = k < n ? __ldcg(table + k) : make_int4(0, 0, 0, 0);
+    for (; k < n; k += G) {
+        int4 nxt = (k + G < n) ? __ldcg(table + k + G) : make_int4(0, 0, 0, 0);
         if (cur.y > 0) gather_list<THREADS>(p.col, p.vec_end, cur.x, cur.y, cur.z, 0u, threadIdx.x, sink, pol);
         cur = nxt;
     }
-    k = global_warp();
-    cur = k < nw ? __ldcg(wtable + k) : make_int4(0, 0, 0, 0);
-    for (; k < nw; k += W) {
-        const int4 nxt = k + W < nw ? __ldcg(wtable + k + W) : make_int4(0, 0, 0, 0);
+}
+
+// Warp chunk phase: warp w of the grid streams warp chunks w, w + W, ...
+template <class Sink>
+__device__ __forceinline__ void gather_wchunks(const BfsParams &p, const int4 *table, unsigned n, const Sink &sink,
+                                               uint64_t pol) {
+    if (n > (unsigned)p.wchunk_cap) n = p.wchunk_cap;
+    const unsigned W = grid_warps();
+    unsigned k = global_warp();
+    int4 cur = k < n ? __ldcg(table + k) : make_int4(0, 0, 0, 0);
+    for (; k < n; k += W) {
+        int4 nxt = (k + W < n) ? __ldcg(table + k + W) : make_int4(0, 0, 0, 0);
         if (cur.y > 0) gather_list<32>(p.col, p.vec_end, cur.x, cur.y, cur.z, 0u, lane_id(), sink, pol);
         cur = nxt;
     }
@@ -373,31 +380,32 @@ __device__ __forceinline__ void gather_whole_chunks(const BfsParams &p, const in
 // are cut into slices of 128 edges, one 16-byte load per lane, that go to the
 // grid's warps in turn.  Slices past a chunk's end are empty and cost one
 // descriptor read.  Larger tables, where they would be most of the work, go
-// out as whole chunks.  So do those of predecessor searches, unless every warp
+// out as whole chunks.  So do those of predecessor searches unless every warp
 // has at most one slice: which of a vertex's possible parents is recorded
-// depends on the order in which the lists are streamed, and callers that
-// compare parent arrays see it change (the slices changed 1.4% of the parents
-// on R-MAT scale 18, against 0.6% from run to run).
+// depends on the order and pace at which the lists are streamed, and callers
+// that compare parent arrays see it change (the slices changed 1.4% of the
+// parents on R-MAT scale 18, against 0.6% from run to run).
 template <int THREADS, bool MP, class Sink>
 __device__ __forceinline__ void gather_chunk_tables(const BfsParams &p, const int4 *ctable, unsigned nch,
                                                     const int4 *wtable, unsigned nw, const Sink &sink,
                                                     uint64_t pol) {
     constexpr unsigned SLICE = 128;
-    constexpr unsigned CS = chunk_edges<THREADS>() / SLICE, WS = WARP_CHUNK / SLICE;  // powers of two
+    constexpr unsigned CS = chunk_edges<THREADS>() / SLICE, WS = WARP_CHUNK / SLICE;
     if (nch > (unsigned)p.chunk_cap) nch = p.chunk_cap;
     if (nw > (unsigned)p.wchunk_cap) nw = p.wchunk_cap;
-    const unsigned W = grid_warps();
     const unsigned long long slices = (unsigned long long)nch * CS + (unsigned long long)nw * WS;
-    if (MP ? slices > (unsigned long long)W : nch >= gridDim.x || nw >= W) {
-        gather_whole_chunks<THREADS>(p, ctable, nch, wtable, nw, sink, pol);
+    if (MP ? slices > (unsigned long long)grid_warps() : nch >= gridDim.x || nw >= unsigned(grid_warps())) {
+        gather_chunks<THREADS>(p, ctable, nch, sink, pol);
+        gather_wchunks(p, wtable, nw, sink, pol);
         return;
     }
-    const unsigned nc = nch * CS, n = nc + nw * WS;  // below W * (CS + WS)
-    for (unsigned k = global_warp(); k < n; k += W) {
-        const int4 ch = __ldcg(k < nc ? ctable + k / CS : wtable + (k - nc) / WS);
-        const int a = (ch.x & ~3) + int((k < nc ? k % CS : (k - nc) % WS) * SLICE);
-        const int s0 = max(a, ch.x), e0 = min(a + int(SLICE), ch.x + ch.y);
+    for (unsigned w = global_warp(); w < slices; w += grid_warps()) {
+        const int4 ch = w < nch * CS ? __ldcg(ctable + w / CS) : __ldcg(wtable + (w - nch * CS) / WS);
+        const unsigned k = w < nch * CS ? w % CS : (w - nch * CS) % WS;
+        const int a0 = (ch.x & ~3) + int(k * SLICE);
+        const int s0 = max(a0, ch.x), e0 = min(a0 + int(SLICE), ch.x + ch.y);
         if (e0 > s0) gather_list<32>(p.col, p.vec_end, s0, e0 - s0, ch.z, 0u, lane_id(), sink, pol);
+        if (MP) return;
     }
 }
 
@@ -532,34 +540,40 @@ __device__ __forceinline__ void gather_windows4(const BfsParams &p, WarpSmem<MP>
     }
 }
 
+// Frontier vertices per lane of a warp tile: 4 (tiles of WINDOW vertices, row
+// ranges and lists of four vertices per lane in flight together) once a level
+// has at least two such tiles per warp of the grid, else 1 (tiles of 32), so
+// that a small level still gives every warp of the grid a tile.
+__device__ __forceinline__ unsigned vertices_per_lane(unsigned L) {
+    return (unsigned long long)L >= 2ull * WINDOW * unsigned(grid_warps()) ? 4u : 1u;
+}
+
 // Queue entries per warp tile of a level of L entries, a power of two: WINDOW
-// (4 per lane, their row ranges and lists in flight together) once a level
-// has two such tiles per warp of the grid; below, one tile per warp, of at
-// most `small` entries, so that the lists of a tile's vertices, which its warp
-// streams window after window in a chain, spread over the grid's idle warps:
-// on a random graph of mean degree 16 a level of 355 edges took 20.9 us in 3
-// tiles of 128 and takes 7.2 us in 45 of 8.  Not below p.tile_min entries,
-// about one window of edges at the graph's mean degree, because each tile
-// makes a queue reservation of its own (lattices, short lists).  Predecessor
-// searches keep tiles of `small` for the order's sake (gather_chunk_tables).
-template <bool MP>
+// once a level has two such tiles per warp of the grid; below, one tile per
+// warp, of at most `small` entries, so that the lists of a tile's vertices,
+// which its warp streams window after window in a chain, spread over the
+// grid's idle warps: on a random graph of mean degree 16 a level of 355 edges
+// took 20.9 us in 3 tiles of 128 and takes 7.2 us in 45 of 8.  Not below
+// p.tile_min entries, about one window of edges at the graph's mean degree,
+// because each tile makes a queue reservation of its own (lattices, short
+// lists).
 __device__ __forceinline__ unsigned tile_width(const BfsParams &p, unsigned L, unsigned small) {
     const unsigned W = unsigned(grid_warps());
-    if ((unsigned long long)L >= 2ull * WINDOW * W) return unsigned(WINDOW);
-    if (MP) return small;
+    if (vertices_per_lane(L) == 4u) return unsigned(WINDOW);
     const unsigned want = max((L + W - 1u) / W, p.tile_min);
     return min(small, 1u << (32 - __clz(int(want) - 1)));
 }
 
 // Loads the frontier vertices of warp tile t (tiles of tw entries) from q_in;
 // bit j of the result marks v[j].
+template <bool MP>
 __device__ __forceinline__ unsigned load_tile(const int *q_in, unsigned L, unsigned t, unsigned tw, int (&v)[4]) {
     unsigned sel = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const unsigned at = unsigned(j) * 32u + lane_id(), idx = t * tw + at;
         v[j] = -1;
-        if (at < tw && idx < L) {
+        if ((MP ? unsigned(j) * 32u : at) < tw && idx < L) {
             v[j] = ld_cg(q_in + idx);
             sel |= 1u << j;
         }
@@ -980,7 +994,7 @@ __device__ void ec_level(const BfsParams &p, int it, unsigned L, unsigned nch, u
     gather_chunk_tables<THREADS, MP>(p, p.chunks[it & 1], nch, p.wchunks[it & 1], nwch, sink, pol);
     WarpSmem<MP> &ws = sm.w[threadIdx.x >> 5];
     const int *q_in = p.queue[it & 1];
-    const unsigned tw = tile_width<MP>(p, L, 32u);
+    const unsigned tw = MP ? 32u * vertices_per_lane(L) : tile_width(p, L, 32u);
     const unsigned ntiles = (L + tw - 1u) / tw;
     const unsigned grab = tile_grab(ntiles);
     const unsigned nruns = (ntiles + grab - 1) / grab;
@@ -988,7 +1002,7 @@ __device__ void ec_level(const BfsParams &p, int it, unsigned L, unsigned nch, u
         const unsigned t0 = r * grab;
         for (unsigned t = t0; t < t0 + grab && t < ntiles; t++) {
             int v[4], st[4], ln[4];
-            const unsigned sel = load_tile(q_in, L, t, tw, v);
+            const unsigned sel = load_tile<MP>(q_in, L, t, tw, v);
             const unsigned has = row_ranges4(p, sel, v, st, ln);
             gather_windows4<MP>(p, ws, has, st, ln, v, sink, pol);
         }
@@ -1029,10 +1043,13 @@ struct alignas(16) WarpStage {
     unsigned long long bar[2];  // mbarriers: bar[b] completes when buf[b] has landed
 };
 
-// One bottom-up step: visited-mask words w0 .. w0 + BU_WORDS - 1.
-template <int THREADS, bool MP>
-__device__ __forceinline__ void bu_step(const BfsParams &p, int it, unsigned w0, unsigned nwords, WarpSmem<MP> &ws,
-                                        int *q_out, unsigned *qlen_out, const BuStage *sg) {
+// One bottom-up step: visited-mask words w0 .. w0 + BU_WORDS - 1.  it: the
+// depth of the parents looked for; q: the ring phase it runs as.  PLACE: long
+// lists of the discovered vertices go to phase q + 1's chunk tables
+// (expand-contract); else every discovered vertex goes to the queue.
+template <int THREADS, bool MP, bool PLACE>
+__device__ __forceinline__ void bu_step(const BfsParams &p, int it, int q, unsigned w0, unsigned nwords,
+                                        WarpSmem<MP> &ws, int *q_out, unsigned *qlen_out, const BuStage *sg) {
     Counters *c = p.ctr;
     const int lane = lane_id();
     unsigned mw[BU_WORDS];
@@ -1225,7 +1242,8 @@ __device__ __forceinline__ void bu_step(const BfsParams &p, int it, unsigned w0,
         }
     }
     count_discovered(ws, nfound, dfound);
-    const unsigned placed = place4<chunk_edges<THREADS>()>(p, it + 1, found, st, ln, v);
+    unsigned placed = 0u;
+    if constexpr (PLACE) placed = place4<chunk_edges<THREADS>()>(p, q + 1, found, st, ln, v);
     stage4(ws, found & ~placed, v, q_out, qlen_out, p.qcap, &c->error);
 }
 
@@ -1278,12 +1296,12 @@ __device__ __forceinline__ bool bu_stage_wait(const BfsParams &p, WarpStage *stg
 // open: an estimate of the vertices still unvisited.  stg (a warp's stage
 // buffers, or NULL) stages each step's row offsets, keys and mask words one
 // step ahead with bulk copies; phase is their mbarriers' parity state.
-template <int THREADS, bool MP>
-__device__ void bu_level(const BfsParams &p, int it, Smem<THREADS, MP> &sm, unsigned open, WarpStage *stg,
+template <int THREADS, bool MP, bool PLACE>
+__device__ void bu_level(const BfsParams &p, int it, int q, Smem<THREADS, MP> &sm, unsigned open, WarpStage *stg,
                          unsigned &phase) {
     Counters *c = p.ctr;
-    int *q_out = p.queue[(it + 1) & 1];
-    unsigned *qlen_out = &c->qlen[(it + 1) & 3];
+    int *q_out = p.queue[(q + 1) & 1];
+    unsigned *qlen_out = &c->qlen[(q + 1) & 3];
     WarpSmem<MP> &ws = sm.w[threadIdx.x >> 5];
     const unsigned nwords = (unsigned(p.nodes) + 31u) >> 5;
     const unsigned nsteps = (nwords + BU_WORDS - 1) / BU_WORDS;
@@ -1298,8 +1316,8 @@ __device__ void bu_level(const BfsParams &p, int it, Smem<THREADS, MP> &sm, unsi
     if (!stg) {
         for (unsigned step = global_warp(); step < nsteps;) {
             unsigned nxt = 0;
-            if (dynamic && lane_id() == 0) nxt = atomicAdd(&c->steal[it & 3], 1u);
-            bu_step<THREADS, MP>(p, it, step * BU_WORDS, nwords, ws, q_out, qlen_out, nullptr);
+            if (dynamic && lane_id() == 0) nxt = atomicAdd(&c->steal[q & 3], 1u);
+            bu_step<THREADS, MP, PLACE>(p, it, q, step * BU_WORDS, nwords, ws, q_out, qlen_out, nullptr);
             step = dynamic ? W + __shfl_sync(FULL, nxt, 0) : step + W;
         }
     } else {
@@ -1311,21 +1329,21 @@ __device__ void bu_level(const BfsParams &p, int it, Smem<THREADS, MP> &sm, unsi
         if (cur < nsteps) {
             bu_prefetch(p, cur, stg, 0);
             unsigned t = 0;
-            if (dynamic && lane_id() == 0) t = atomicAdd(&c->steal[it & 3], 1u);
+            if (dynamic && lane_id() == 0) t = atomicAdd(&c->steal[q & 3], 1u);
             nxt = dynamic ? W + __shfl_sync(FULL, t, 0) : cur + W;
             if (nxt < nsteps) bu_prefetch(p, nxt, stg, 1);
         }
         while (cur < nsteps) {
             unsigned t = 0;
             const bool more = nxt < nsteps;
-            if (more && dynamic && lane_id() == 0) t = atomicAdd(&c->steal[it & 3], 1u);
+            if (more && dynamic && lane_id() == 0) t = atomicAdd(&c->steal[q & 3], 1u);
             if (!bu_stage_wait(p, stg, b, phase)) {
                 // Abandon the level: wait (bounded again) for the copies still
                 // in flight into the other buffer, then leave.
                 if (more) bu_stage_wait(p, stg, b ^ 1, phase);
                 break;
             }
-            bu_step<THREADS, MP>(p, it, cur * BU_WORDS, nwords, ws, q_out, qlen_out, &stg->buf[b]);
+            bu_step<THREADS, MP, PLACE>(p, it, q, cur * BU_WORDS, nwords, ws, q_out, qlen_out, &stg->buf[b]);
             unsigned nxt2 = nsteps;
             if (more) nxt2 = dynamic ? W + __shfl_sync(FULL, t, 0) : nxt + W;
             if (nxt2 < nsteps) bu_prefetch(p, nxt2, stg, b);
@@ -1335,7 +1353,7 @@ __device__ void bu_level(const BfsParams &p, int it, Smem<THREADS, MP> &sm, unsi
         }
     }
     stage_drain(ws, q_out, qlen_out, p.qcap, &c->error);
-    flush_discovered(p, ws, it + 1);
+    flush_discovered(p, ws, q + 1);
 }
 
 // Edge-frontier phase input: warp tiles of tw elements (tile_width; coalesced),
@@ -1353,7 +1371,7 @@ __device__ __forceinline__ void edge_tiles(const int *q_in, const int *pq_in, un
             const unsigned at = unsigned(j) * 32u + lane_id(), idx = t * tw + at;
             u[j] = -1;
             pr[j] = 0;
-            if (at < tw && idx < L) {
+            if ((MP || at < tw) && idx < L) {  // predecessor searches: full tiles
                 valid |= 1u << j;
                 u[j] = ld_cg(q_in + idx);
                 if (MP) pr[j] = ld_cg(pq_in + idx);
@@ -1370,7 +1388,7 @@ __device__ void ce_level(const BfsParams &p, int it, int q, unsigned L, unsigned
                          Smem<THREADS, MP> &sm, uint64_t pol) {
     ContractExpandSink<THREADS, MP> sink{p, sm, it, q, pol, probe_level(phase_work<THREADS>(L, 1u, nch, nwch))};
     gather_chunk_tables<THREADS, MP>(p, p.chunks[q & 1], nch, p.wchunks[q & 1], nwch, sink, pol);
-    edge_tiles<MP>(p.queue[q & 1], p.pred_queue[q & 1], L, tile_width<MP>(p, L, unsigned(WINDOW)), sink);
+    edge_tiles<MP>(p.queue[q & 1], p.pred_queue[q & 1], L, MP ? unsigned(WINDOW) : tile_width(p, L, unsigned(WINDOW)), sink);
     sink.drain();
 }
 
@@ -1396,7 +1414,7 @@ __device__ void tp_expand(const BfsParams &p, int qi, unsigned L, bool cull, Sme
     WarpSmem<MP> &ws = sm.w[threadIdx.x >> 5];
     const FilterSink<THREADS, MP> out{p, sm, p.queue[nq], p.pred_queue[nq], &c->qlen[(qi + 1) & 3]};
     const int *q_in = p.queue[qi & 1];
-    const unsigned tw = tile_width<MP>(p, L, 32u);
+    const unsigned tw = MP ? 32u * vertices_per_lane(L) : tile_width(p, L, 32u);
     const unsigned ntiles = (L + tw - 1u) / tw;
     const unsigned grab = tile_grab(ntiles);
     const unsigned nruns = (ntiles + grab - 1) / grab;
@@ -1404,7 +1422,7 @@ __device__ void tp_expand(const BfsParams &p, int qi, unsigned L, bool cull, Sme
         const unsigned t0 = r * grab;
         for (unsigned t = t0; t < t0 + grab && t < ntiles; t++) {
             int v[4], st[4], ln[4];
-            const unsigned sel = load_tile(q_in, L, t, tw, v);
+            const unsigned sel = load_tile<MP>(q_in, L, t, tw, v);
             const unsigned has = row_ranges4(p, sel, v, st, ln);
             if (cull || p.count_raw) count_raw(&ws.raw_n, has, ln);
             const unsigned placed = place4<chunk_edges<THREADS>()>(p, qi + 1, has, st, ln, v);
@@ -1777,7 +1795,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS(THREADS)) ec_fused_kernel(
                 if (!grid_barrier(c, p.wait_ns, &sm.flag)) break;
             }
             const unsigned done = dir.visited + lc.zmarked;
-            bu_level<THREADS, MP>(p, it, sm, done < unsigned(p.nodes) ? unsigned(p.nodes) - done : 0u, stg, phase);
+            bu_level<THREADS, MP, true>(p, it, it, sm, done < unsigned(p.nodes) ? unsigned(p.nodes) - done : 0u, stg, phase);
         } else {
             ec_level<THREADS, MP>(p, it, L, nch, nw, sm, pol);
         }
@@ -1943,6 +1961,100 @@ __device__ void ce_flat_level(const BfsParams &p, int it, int q, unsigned L, Sme
     }
 }
 
+// The bottom-up levels of the edge-frontier strategies (depth labels of a
+// symmetric graph; DirectionChoice's rule on the levels' raw edge frontiers).
+// At level it, ring phase q, the edge frontier in the queue and the chunk
+// tables is left unread: bottom-up levels label the vertices of depth it, it +
+// 1, ... and queue them, until the rule turns back; then one two-phase expand
+// turns the last of them into the edge frontier the caller's next level
+// contracts.  On R-MAT scale 21 contract-expand spent 715 us of a search's 790
+// in the two levels that contract 60 M edges of mostly visited vertices;
+// bottom-up the search takes 117 us.
+struct EdgeState {
+    int it, q, log;      // level, ring phase, level-log index
+    LevelCounts lc;      // counts of ring phase q
+    bool ended;          // the search is over: its iteration count is `it`
+    bool failed;         // a barrier ended on an error
+    bool top_down = false;  // level it's direction is decided: bottom-up levels turned back before it
+
+    // Whether level it runs bottom-up (every CTA decides alike).
+    __device__ __forceinline__ bool bottom_up(const BfsParams &p, DirectionChoice &dir) {
+        if (!p.do_alpha) return false;
+        const bool decided = top_down;
+        top_down = false;
+        return !decided && dir.next(p, 0u, lc.raw) && it > 0;
+    }
+};
+
+// records(raw): whether the level logs and counts as two phases (a contract
+// and an expand record, no count of a level that discovers nothing) or as one.
+template <int THREADS, class Records>
+__device__ void edge_bottom_up(const BfsParams &p, EdgeState &s, DirectionChoice &dir, Smem<THREADS, false> &sm,
+                               BusyClock &clk, uint64_t pol, const Records &two_records) {
+    Counters *c = p.ctr;
+    unsigned phase = 0, zmarked = 0;
+    unsigned long long raw = s.lc.raw;
+    unsigned nch = s.lc.nch, nw = s.lc.nw;
+    s.ended = s.failed = false;
+    for (;;) {
+        const bool two = two_records(raw);
+        if (leader()) {
+            ring_prepare(c, s.q);
+            atomicAdd(&c->total_queued, raw);
+            log_phase(p, s.log, unsigned(raw), nch, nw, 1u);
+        }
+        const unsigned done = dir.visited + zmarked;
+        bu_level<THREADS, false, false>(p, s.it - 1, s.q, sm, done < unsigned(p.nodes) ? unsigned(p.nodes) - done : 0u,
+                                        nullptr, phase);
+        clk.stop(p);
+        log_work_end(p, s.log);
+        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, true))) {
+            s.failed = true;
+            return;
+        }
+        clk.start(p);
+        s.lc = sm.lc;
+        zmarked = s.lc.zmarked;
+        s.q++;
+        s.log++;
+        if (s.lc.nf == 0u) {  // nothing of depth it: one-phase levels count this one, two-phase ones do not
+            if (!two) s.it++;
+            s.ended = true;
+            return;
+        }
+        s.it++;
+        const bool stay = dir.next(p, s.lc.nf, s.lc.mf);
+        if (two && stay) {  // no expand: its record starts and ends here
+            if (leader()) {
+                log_phase(p, s.log, s.lc.nf, 0u, 0u);
+                if (p.levels && s.log < p.level_cap) p.levels[s.log].t_work_end = p.levels[s.log].t_start;
+            }
+            s.log++;
+        }
+        if (!stay) {
+            if (leader()) {
+                ring_prepare(c, s.q);
+                if (two) log_phase(p, s.log, s.lc.nf, 0u, 0u);
+            }
+            tp_expand<THREADS, false>(p, s.q, s.lc.L, gather_cull(s.lc.mf), sm, pol);
+            clk.stop(p);
+            if (two) log_work_end(p, s.log);
+            if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) {
+                s.failed = true;
+                return;
+            }
+            clk.start(p);
+            s.lc = sm.lc;
+            s.q++;
+            if (two) s.log++;
+            s.top_down = true;
+            return;
+        }
+        raw = s.lc.mf;
+        nch = nw = 0u;
+    }
+}
+
 // Whether a full-grid contract-expand level runs ce_flat_level: no chunked
 // lists, at most p.flat_max queued edges, and at most one per grid thread.
 // A second round of the latency-first body costs more than the tiled body
@@ -1962,35 +2074,47 @@ __device__ __forceinline__ void ce_search(const BfsParams &p) {
     const uint64_t pol = column_policy(p);
     Counters *c = p.ctr;
     BusyClock clk;
-    int it = __ldcg(&c->resume);
-    LevelCounts lc = read_counts(c, it, false, sm);
+    DirectionChoice dir;
+    EdgeState s;
+    s.it = s.q = __ldcg(&c->resume);  // q: the level, less those that bottom-up levels and their expand shift it by
+    s.lc = read_counts(c, s.q, false, sm);
     // A narrow launch before this one raised an error: no level runs.  (A CTA
     // may also see an error another CTA raised in its first level and leave
     // at once; the others' grid barrier ends on the error.)
     const bool failed = ld_relaxed_gpu(&c->error) != 0u;
     for (; !failed;) {
         clk.start(p);
-        const unsigned L = lc.L, nch = lc.nch, nw = lc.nw;
+        const unsigned L = s.lc.L, nch = s.lc.nch, nw = s.lc.nw;
         // raw: the edge frontier before the gather-time cull, so the loop runs
         // (and counts) the levels the reference runs, the last one empty here
-        if (stop_level_loop(p, it, L + nch + nw + lc.raw)) break;
+        if (stop_level_loop(p, s.it, L + nch + nw + s.lc.raw)) break;
+        if constexpr (edge_switch(THREADS, MP)) {
+            if (s.bottom_up(p, dir)) {
+                s.log = s.it;
+                edge_bottom_up<THREADS>(p, s, dir, sm, clk, pol, [](unsigned long long) { return false; });
+                clk.stop(p);
+                if (s.ended || s.failed) break;
+                continue;
+            }
+        }
         if (leader()) {
-            ring_prepare(c, it);
-            atomicAdd(&c->total_queued, (unsigned long long)lc.raw);
-            log_phase(p, it, lc.raw ? lc.raw : L, nch, nw);
+            ring_prepare(c, s.q);
+            atomicAdd(&c->total_queued, (unsigned long long)s.lc.raw);
+            log_phase(p, s.it, s.lc.raw ? s.lc.raw : L, nch, nw);
         }
         if (flat_level<THREADS>(p, L, nch + nw))
-            ce_flat_level<THREADS, MP>(p, it, it, L, sm);
+            ce_flat_level<THREADS, MP>(p, s.it, s.q, L, sm);
         else
-            ce_level<THREADS, MP>(p, it, it, L, nch, nw, sm, pol);
+            ce_level<THREADS, MP>(p, s.it, s.q, L, nch, nw, sm, pol);
         clk.stop(p);
-        log_work_end(p, it);
-        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, it + 1, false))) break;
-        lc = sm.lc;
-        it++;
+        log_work_end(p, s.it);
+        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) break;
+        s.lc = sm.lc;
+        s.q++;
+        s.it++;
     }
     clk.flush(p);
-    finish_search(p, it, it);
+    finish_search(p, s.it, s.it);
 }
 
 // A level's counts from counters in shared memory (a narrow launch's); dir:
@@ -2362,42 +2486,57 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS(THREADS)) tp_fused_kernel(
     // search (resume -1: nothing left to do).
     const int resume = __ldcg(&c->resume);
     if (resume < 0) return;
-    int it = resume, qi = 2 * resume;
-    LevelCounts lc = read_counts(c, qi, false, sm);
+    DirectionChoice dir;
+    EdgeState s;  // q: the ring phase (2 * it until bottom-up levels, which take one phase, shift it)
+    s.it = resume;
+    s.q = 2 * resume;
+    s.lc = read_counts(c, s.q, false, sm);
+    int end_log = 2 * s.it + 1;  // where the end marker goes
     const bool failed = ld_relaxed_gpu(&c->error) != 0u;  // as ce_search
     for (; !failed;) {
         clk.start(p);
-        unsigned L = lc.L;
-        const unsigned nch = lc.nch, nw = lc.nw;
-        if (stop_level_loop(p, it, L + nch + nw + lc.raw)) break;
-        const bool cull = gather_cull(level_edges<THREADS>(lc));
-        if (leader()) {
-            ring_prepare(c, qi);
-            atomicAdd(&c->total_queued, (unsigned long long)lc.raw);
-            log_phase(p, qi, lc.raw ? lc.raw : L, nch, nw);
+        const unsigned L = s.lc.L, nch = s.lc.nch, nw = s.lc.nw;
+        end_log = 2 * s.it + 1;
+        if (stop_level_loop(p, s.it, L + nch + nw + s.lc.raw)) break;
+        if constexpr (edge_switch(THREADS, MP)) {
+            if (s.bottom_up(p, dir)) {
+                s.log = 2 * s.it;
+                edge_bottom_up<THREADS>(p, s, dir, sm, clk, pol, [](unsigned long long) { return true; });
+                clk.stop(p);
+                if (s.ended) end_log = 2 * s.it + 2;
+                if (s.ended || s.failed) break;
+                continue;
+            }
         }
-        tp_contract<THREADS, MP>(p, it, qi, L, nch, nw, sm, pol);
+        const bool cull = gather_cull(level_edges<THREADS>(s.lc));
+        if (leader()) {
+            ring_prepare(c, s.q);
+            atomicAdd(&c->total_queued, (unsigned long long)s.lc.raw);
+            log_phase(p, 2 * s.it, s.lc.raw ? s.lc.raw : L, nch, nw);
+        }
+        tp_contract<THREADS, MP>(p, s.it, s.q, L, nch, nw, sm, pol);
         clk.stop(p);
-        log_work_end(p, qi);
-        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, qi + 1, false))) break;
+        log_work_end(p, 2 * s.it);
+        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) break;
         clk.start(p);
-        qi++;
-        L = sm.lc.L;
-        if (L == 0u) break;  // no vertex discovered: the reference stops without ++
+        s.q++;
+        end_log = 2 * s.it + 2;
+        const unsigned Lv = sm.lc.L;
+        if (Lv == 0u) break;  // no vertex discovered: the reference stops without ++
         if (leader()) {
-            ring_prepare(c, qi);
-            log_phase(p, qi, L, 0u, 0u);
+            ring_prepare(c, s.q);
+            log_phase(p, 2 * s.it + 1, Lv, 0u, 0u);
         }
-        tp_expand<THREADS, MP>(p, qi, L, cull, sm, pol);
+        tp_expand<THREADS, MP>(p, s.q, Lv, cull, sm, pol);
         clk.stop(p);
-        log_work_end(p, qi);
-        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, qi + 1, false))) break;
-        lc = sm.lc;
-        qi++;
-        it++;
+        log_work_end(p, 2 * s.it + 1);
+        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) break;
+        s.lc = sm.lc;
+        s.q++;
+        s.it++;
     }
     clk.flush(p);
-    finish_search(p, it, qi + 1);
+    finish_search(p, s.it, end_log);
 }
 
 // Hybrid (the reference's EnactorHybrid, enactor_hybrid.cuh:279-555): a level
@@ -2419,57 +2558,71 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS(THREADS)) hy_fused_kernel(
     BusyClock clk;
     // A narrow launch (contract-expand levels on one cluster, where the ring
     // phase is the level) may have run the first levels.
-    int it = __ldcg(&c->resume), q = it;
-    LevelCounts lc = read_counts(c, q, false, sm);
+    DirectionChoice dir;
+    EdgeState s;
+    s.it = s.q = s.log = __ldcg(&c->resume);
+    s.lc = read_counts(c, s.q, false, sm);
+    const auto log_at = [&s] { return edge_switch(THREADS, MP) ? s.log : s.q; };  // they part at bottom-up levels
     const bool failed = ld_relaxed_gpu(&c->error) != 0u;  // as ce_search
     for (; !failed;) {
         clk.start(p);
-        unsigned L = lc.L;
-        const unsigned nch = lc.nch, nw = lc.nw;
-        if (stop_level_loop(p, it, L + nch + nw + lc.raw)) break;
+        const unsigned L = s.lc.L, nch = s.lc.nch, nw = s.lc.nw;
+        if (stop_level_loop(p, s.it, L + nch + nw + s.lc.raw)) break;
+        if constexpr (edge_switch(THREADS, MP)) {
+            if (s.bottom_up(p, dir)) {
+                edge_bottom_up<THREADS>(p, s, dir, sm, clk, pol,
+                                        [saturation](unsigned long long raw) { return raw > saturation; });
+                clk.stop(p);
+                if (s.ended || s.failed) break;
+                continue;
+            }
+        }
         if (leader()) {
-            ring_prepare(c, q);
-            atomicAdd(&c->total_queued, (unsigned long long)lc.raw);
-            log_phase(p, q, lc.raw ? lc.raw : L, nch, nw);
+            ring_prepare(c, s.q);
+            atomicAdd(&c->total_queued, (unsigned long long)s.lc.raw);
+            log_phase(p, log_at(), s.lc.raw ? s.lc.raw : L, nch, nw);
         }
         // the level's edge frontier as the reference counts it (before the gather-time cull)
-        const unsigned long long edges = level_edges<THREADS>(lc);
+        const unsigned long long edges = level_edges<THREADS>(s.lc);
         if (edges <= saturation) {
             if (flat_level<THREADS>(p, L, nch + nw))
-                ce_flat_level<THREADS, MP>(p, it, q, L, sm);
+                ce_flat_level<THREADS, MP>(p, s.it, s.q, L, sm);
             else
-                ce_level<THREADS, MP>(p, it, q, L, nch, nw, sm, pol);
+                ce_level<THREADS, MP>(p, s.it, s.q, L, nch, nw, sm, pol);
             clk.stop(p);
-            log_work_end(p, q);
-            if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, q + 1, false))) break;
-            lc = sm.lc;
-            q++;
-            it++;
+            log_work_end(p, log_at());
+            if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) break;
+            s.lc = sm.lc;
+            s.q++;
+            s.log++;
+            s.it++;
             continue;
         }
         const bool cull = gather_cull(edges);
-        tp_contract<THREADS, MP>(p, it, q, L, nch, nw, sm, pol);
+        tp_contract<THREADS, MP>(p, s.it, s.q, L, nch, nw, sm, pol);
         clk.stop(p);
-        log_work_end(p, q);
-        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, q + 1, false))) break;
+        log_work_end(p, log_at());
+        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) break;
         clk.start(p);
-        q++;
-        L = sm.lc.L;
-        if (L == 0u) break;  // no vertex discovered: stop without ++, as two-phase does
+        s.q++;
+        s.log++;
+        const unsigned Lv = sm.lc.L;
+        if (Lv == 0u) break;  // no vertex discovered: stop without ++, as two-phase does
         if (leader()) {
-            ring_prepare(c, q);
-            log_phase(p, q, L, 0u, 0u);
+            ring_prepare(c, s.q);
+            log_phase(p, log_at(), Lv, 0u, 0u);
         }
-        tp_expand<THREADS, MP>(p, q, L, cull, sm, pol);
+        tp_expand<THREADS, MP>(p, s.q, Lv, cull, sm, pol);
         clk.stop(p);
-        log_work_end(p, q);
-        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, q + 1, false))) break;
-        lc = sm.lc;
-        q++;
-        it++;
+        log_work_end(p, log_at());
+        if (!grid_barrier(c, p.wait_ns, &sm.flag, next_counts(&sm.lc, s.q + 1, false))) break;
+        s.lc = sm.lc;
+        s.q++;
+        s.log++;
+        s.it++;
     }
     clk.flush(p);
-    finish_search(p, it, q);
+    finish_search(p, s.it, log_at());
 }
 
 // ---- per-level kernels for the graph-driven (iterative) variants ----------------
@@ -2712,13 +2865,20 @@ __global__ void reset_state_kernel(int *labels, long long n, unsigned *mask, lon
 
 // CSR checks on the device: out[0] = the first row v whose offsets decrease
 // (row[v+1] < row[v]), out[1] = the first entry outside [0, nodes); both stay
-// ~0 when there is none (out must start at ~0).
+// ~0 when there is none (they must start at ~0).  out[2] = the largest degree
+// (it must start at 0).
 __global__ void csr_check_kernel(const int *row_offsets, const int *col, int nodes, long long edges,
                                  unsigned long long *out) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (long long v = t; v < nodes; v += stride)
-        if (__ldg(row_offsets + v + 1) < __ldg(row_offsets + v)) atomicMin(out + 0, (unsigned long long)v);
+    int longest = 0;
+    for (long long v = t; v < nodes; v += stride) {
+        const int len = __ldg(row_offsets + v + 1) - __ldg(row_offsets + v);
+        if (len < 0) atomicMin(out + 0, (unsigned long long)v);
+        longest = max(longest, len);
+    }
+    longest = __reduce_max_sync(FULL, longest);
+    if (lane_id() == 0 && longest > 0) atomicMax(out + 2, (unsigned long long)longest);
     for (long long k = t; k < edges; k += stride)
         if ((unsigned)__ldg(col + k) >= (unsigned)nodes) atomicMin(out + 1, (unsigned long long)k);
 }

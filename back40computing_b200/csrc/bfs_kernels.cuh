@@ -112,6 +112,16 @@ __host__ __device__ constexpr int chunk_edges() { return THREADS * 16; }
 // Edges per warp chunk: four passes of one 16-byte load per lane.
 constexpr int WARP_CHUNK = 512;
 
+// Graphs without a longer list are low-degree graphs (lattices, road
+// networks): their levels are too small for bottom-up sweeps to pay.
+constexpr int LOW_DEGREE = 16;
+
+// Whether the edge-frontier strategies' fused kernels have bottom-up levels:
+// depth labels, 512-thread CTAs.  At 128 and 256 threads (48 registers) the
+// bottom-up body would spill 700 bytes and slow the top-down levels (two-phase
+// on a directed R-MAT scale 20: 300 -> 391 us).
+__host__ __device__ constexpr bool edge_switch(int threads, bool mark_pred) { return threads == 512 && !mark_pred; }
+
 struct KernelConfig {
     int strategy;
     int threads;  // 128, 256 or 512
@@ -140,8 +150,8 @@ cudaError_t launch_heavy_neighbour(const int *row_offsets, const int *col, int n
 cudaError_t launch_reset_state(int *labels, long long nodes, unsigned *mask, long long mask_words,
                                cudaStream_t stream);
 // CSR validity on the device: out[0] = first row whose offsets decrease,
-// out[1] = first column entry outside [0, nodes); ~0 when none.  out[0..1]
-// must start at ~0.
+// out[1] = first column entry outside [0, nodes); ~0 when none; out[2] = the
+// largest degree.  out[0..1] must start at ~0, out[2] at 0.
 cudaError_t launch_csr_check(const int *row_offsets, const int *col, int nodes, long long edges,
                              unsigned long long *out, cudaStream_t stream);
 // Cooperative launch of the persistent kernel that runs every BFS level.

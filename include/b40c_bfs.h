@@ -147,7 +147,7 @@ int b40c_enactor_last_elapsed_ms(b40c_enactor_t *enactor, float *ms);
 int b40c_enactor_set_stream(b40c_enactor_t *enactor, void *stream);
 /* Tuning policy (the reference's compile-time KernelPolicy, kernel_policy.cuh:61-87,
  * WARP_GATHER_THRESHOLD / CTA_GATHER_THRESHOLD): cta_threads in {128,256,512}
- * (default 512 for expand-contract, 256 for the others);
+ * (default 512);
  * lists of at least cta_gather_threshold edges (default 1024) are cut into
  * chunks of 16 * cta_threads edges, each gathered by a whole CTA; lists of at
  * least warp_gather_threshold edges (default 128 for expand-contract, 64 for
@@ -179,18 +179,20 @@ int b40c_enactor_level_log(b40c_enactor_t *enactor, int max_records, int64_t *t_
  * reference. */
 int b40c_enactor_level_times(b40c_enactor_t *enactor, int max_records, int64_t *t_start_ns,
                              int64_t *t_work_end_ns, int *count);
-/* Direction-optimizing expand-contract (an addition; the reference's
- * expand-contract is top-down only): a level runs bottom-up -- each unvisited
- * vertex scans its list for a parent in the frontier -- once the frontier's
- * edges exceed the unvisited vertices' edges / alpha, and returns to top-down
- * once the frontier holds fewer than nodes / beta vertices and shrinks
- * (Beamer, Asanovic and Patterson, SC 2012).  Defaults alpha = 14, beta = 24;
- * alpha = 0 turns it off.  It applies to fused searches on symmetric graphs
- * held on the device (not stream_from_host), checked once per graph; other
- * searches stay top-down.  Depth
- * labels, search depth and total_queued are those of top-down; predecessor
- * labels are valid predecessors (bottom-up levels record the parent they
- * find). */
+/* Direction switch (an addition; the reference's searches are top-down
+ * only): a level runs bottom-up -- each unvisited vertex scans its list for a
+ * parent in the frontier -- once the frontier's edges exceed the unvisited
+ * vertices' edges / alpha, and returns to top-down once the frontier holds
+ * fewer than nodes / beta vertices and shrinks (Beamer, Asanovic and
+ * Patterson, SC 2012).  It applies to fused searches on symmetric graphs held
+ * on the device (not stream_from_host), checked once per graph; other searches
+ * stay top-down.  Depth labels, search depth and total_queued are those of
+ * top-down; predecessor labels are valid predecessors (bottom-up levels record
+ * the parent they find).  Every strategy starts with alpha = 14, beta = 24;
+ * alpha = 0 turns the switch off.  Values above 0 can be set for
+ * expand-contract only; the other strategies switch with the defaults, for
+ * depth labels, with 512-thread CTAs, on graphs with a list of more than 16
+ * edges. */
 int b40c_enactor_set_direction_optimizing(b40c_enactor_t *enactor, int alpha, int beta);
 /* Spin limit of every device-side wait (grid barrier), in microseconds. */
 int b40c_enactor_set_wait_limit_us(b40c_enactor_t *enactor, long long us);
