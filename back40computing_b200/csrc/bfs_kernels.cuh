@@ -127,6 +127,7 @@ struct KernelConfig {
     int threads;  // 128, 256 or 512
     bool mark_pred;
     bool stage_bu = false;  // the launch carries the bottom-up stage buffers (BfsParams::stage_bu)
+    int low_degree = -1;    // a low-degree search (low_degree.cu): its graph's largest degree; -1: not one
 };
 
 // Enqueues the per-search initialisation (counters, source) on stream.
@@ -169,6 +170,24 @@ cudaError_t launch_narrow(const BfsParams &p, const KernelConfig &kc, int team, 
 // sets the loop condition on the device.  p.cond_handle is filled in.
 cudaError_t build_level_graph(BfsParams &p, const KernelConfig &kc, int grid,
                               cudaGraphExec_t *exec, cudaGraph_t *graph);
+// Low-degree searches (low_degree.cu): depth labels, fused, no list of more
+// than LOW_DEGREE edges, nodes < LF_NODES.
+constexpr int LF_TEAM = 16;                  // CTAs of a cluster
+constexpr unsigned LF_STARTS = 1u << 20;     // entries of the row-start side queues
+constexpr unsigned LF_COUNTS = 2 * 512;      // entries of LowDegreeParams::counts
+constexpr long long LF_NODES = 1ll << 27;    // ids share a word with the list length
+struct LowDegreeParams {
+    int *starts[2];  // LF_STARTS row starts beside the first entries of queue[0] and queue[1]
+    uint2 *counts;   // LF_COUNTS: by level parity, what each CTA discovered (vertices, their edges)
+    int strategy;    // whose statistics and level log the search reports
+    int max_degree;
+};
+// Which kernel serves lists of at most max_degree edges (4, 8 or 16 lanes a list).
+inline int low_degree_class(int max_degree) { return max_degree <= 4 ? 0 : max_degree <= 8 ? 1 : 2; }
+// Largest co-resident grid, a multiple of LF_TEAM (0: no cluster fits).
+cudaError_t low_degree_grid_limit(int max_degree, int *grid);
+// The search's two launches: initialisation, then the persistent kernel.
+cudaError_t launch_low_degree(const BfsParams &p, const LowDegreeParams &a, int grid, cudaStream_t stream);
 // Debug/failure-detection probe: a cooperative grid whose barrier expects one
 // more arrival than there are CTAs.  Returns the device error word.
 cudaError_t run_barrier_timeout_probe(int grid, unsigned long long wait_ns, unsigned *error_out);
