@@ -256,7 +256,8 @@ class _Enactor:
                 for i in range(n.value)]
 
     def set_direction_optimizing(self, alpha: int = 14, beta: int = 24) -> None:
-        """Bottom-up levels for fused expand-contract searches (alpha = 0: off)."""
+        """Bottom-up levels of fused searches (alpha = 0: off; other values for
+        expand-contract only, the other strategies run the defaults)."""
         check(lib().b40c_enactor_set_direction_optimizing(self._h, int(alpha), int(beta)))
 
     def set_wait_limit_us(self, us: int) -> None:
@@ -271,7 +272,8 @@ class _Enactor:
         entries run on one cluster of team_ctas CTAs (0: none), and
         (contract-expand, hybrid) full-grid levels of at most grid_frontier
         queued entries run the latency-first level body (0: none).  Both off
-        by default."""
+        by default; depth-label searches of graphs without a list of more than
+        16 edges need neither and ignore both."""
         check(lib().b40c_enactor_set_narrow_levels(self._h, int(team_ctas), int(max_frontier), int(grid_frontier)))
 
     def narrow_team(self) -> int:

@@ -97,6 +97,7 @@ struct b40c_enactor {
     int strategy = B40C_EXPAND_CONTRACT;
     bool instrument = false, debug = false;
     int threads = 256;
+    bool threads_user = false;  // set by the caller, not the default
     int warp_th = 64, cta_th = 1024;
     unsigned cull_flags = CULL_HISTORY;
     unsigned do_alpha = 0, do_beta = 0;  // direction switch (0: top-down only)
@@ -117,11 +118,13 @@ struct b40c_enactor {
     int4 *d_wchunks[2] = {nullptr, nullptr};  // warp chunks
     int chunk_cap = 0;   // entries per CTA chunk table
     int wchunk_cap = 0;  // entries per warp chunk table
-    int *d_starts = nullptr;  // low-degree searches: the two row-start side queues and the CTAs' counts
-    int low_grid[3] = {-1, -1, -1};  // their grid limit (lists of at most 4 / 8 / 16 edges; -1: not asked yet)
+    int low_grid[3] = {-1, -1, -1};  // low-degree searches: the grid limit (lists of at most 4 / 8 / 16 edges; -1: not asked yet)
     LevelRecord *d_levels = nullptr;  // per-level log, when enabled
     bool log_levels = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t dep = nullptr;  // orders the problem's stream and the enactor's
+    int fused_key = -1;         // launch configuration fused_limit was found for
+    int fused_limit = 0;        // largest co-resident grid
     float last_ms = 0.f;
     int last_iteration = 0;
     long long last_total_queued = 0;
@@ -146,6 +149,7 @@ struct b40c_enactor {
 namespace {
 
 constexpr int LEVEL_LOG_CAP = 4096;
+constexpr int CHUNK_ENTRIES_MIN = 512;  // of each chunk table
 
 cudaStream_t problem_stream(b40c_problem *p) { return p->stream ? p->stream : p->own_stream; }
 // The label buffer the last Reset initialised: searches write it, extracts read it.
@@ -336,8 +340,8 @@ int ensure_enactor_buffers(b40c_enactor *e, b40c_problem *p) {
     // edges placed in a table of CH-edge chunks takes at most len / CH + 2
     // entries (CH >= 2048 for CTA chunks, 512 for warp chunks).
     const long long ct = std::max(1, std::max(e->cta_th, e->warp_th)), wt = std::max(1, e->warp_th);
-    long long need = p->edges / chunk_edges<128>() + 2 * (p->edges / ct) + 64;
-    long long wneed = p->edges / WARP_CHUNK + 2 * (p->edges / wt) + 64;
+    long long need = p->edges / chunk_edges<128>() + 2 * (p->edges / ct) + CHUNK_ENTRIES_MIN;
+    long long wneed = p->edges / WARP_CHUNK + 2 * (p->edges / wt) + CHUNK_ENTRIES_MIN;
     need = std::min(need, 1ll << 30);
     wneed = std::min(wneed, 1ll << 30);
     if (e->chunk_cap < need) {
@@ -436,11 +440,8 @@ int enqueue_search(b40c_enactor *e, b40c_problem *p, int src, int max_grid_size,
     // The problem's pending work (Reset) precedes the search.
     cudaStream_t ps = problem_stream(p);
     if (ps != s) {
-        cudaEvent_t dep;
-        CUDA_TRY(cudaEventCreateWithFlags(&dep, cudaEventDisableTiming), "cudaEventCreate");
-        cudaEventRecord(dep, ps);
-        cudaStreamWaitEvent(s, dep, 0);
-        cudaEventDestroy(dep);
+        cudaEventRecord(e->dep, ps);
+        cudaStreamWaitEvent(s, e->dep, 0);
     }
     if (variant < B40C_VARIANT_DEFAULT || variant > B40C_VARIANT_ITERATIVE)
         return set_error(B40C_ERR_INVALID_VALUE, "unknown variant %d", variant);
@@ -466,29 +467,43 @@ int enqueue_search(b40c_enactor *e, b40c_problem *p, int src, int max_grid_size,
     // On low-degree graphs the other strategies stay top-down too (counting
     // their edge frontiers and sweeping the last levels took the 256^3 lattice
     // from 4.5 to 8.0 ms).
-    if (kc.low_degree < 0 && variant == B40C_VARIANT_FUSED && e->do_alpha && !p->mapped &&
-        (e->strategy == B40C_EXPAND_CONTRACT ||
-         (edge_switch(e->threads, p->mark_pred) && p->max_degree > LOW_DEGREE))) {
+    const bool ec = e->strategy == B40C_EXPAND_CONTRACT;
+    bool bottom_up = kc.low_degree < 0 && variant == B40C_VARIANT_FUSED && e->do_alpha && !p->mapped &&
+                     (ec || (edge_switch(e->threads_user ? e->threads : 512, p->mark_pred) &&
+                             p->max_degree > LOW_DEGREE));
+    if (bottom_up) {
         if ((rc = ensure_symmetry_known(p))) return rc;
-        if (p->symmetric == 1) {
-            if (p->mark_pred && p->mask_snap_cap < p->mask_bytes) {
-                cudaFree(p->d_mask_snap);
-                p->d_mask_snap = nullptr;
-                p->mask_snap_cap = 0;
-                CUDA_TRY(cudaMalloc(&p->d_mask_snap, p->mask_bytes), "cudaMalloc visited-mask copy");
-                p->mask_snap_cap = p->mask_bytes;
-            }
-            if ((rc = ensure_heavy_known(p))) return rc;
-            bp.mask_snap = p->d_mask_snap;
-            bp.heavy = p->d_heavy;
-            // the problem's row offsets, mask and keys carry the padding, and
-            // the expand-contract launch the stage buffers
-            kc.stage_bu = e->stage_bu && e->strategy == B40C_EXPAND_CONTRACT;
-            bp.stage_bu = kc.stage_bu ? 1 : 0;
-            bp.do_alpha = e->do_alpha;
-            bp.do_beta = e->do_beta;
-            if (e->strategy != B40C_EXPAND_CONTRACT) bp.count_raw = 1;  // the edge frontiers decide the direction
+        bottom_up = p->symmetric == 1;
+    }
+    // The caller's CTA size, or the default but: two-phase and the hybrid need
+    // 512 threads for bottom-up levels (edge_switch) and are faster with them on
+    // low-degree graphs (predecessors on a lattice: 1824 -> 1528 us), and large
+    // graphs that
+    // expand-contract searches top-down are faster with 256 (directed R-MAT
+    // scale 20: 329 -> 298 us; their largest levels want the warps more than
+    // the registers).
+    if (!e->threads_user && variant == B40C_VARIANT_FUSED) {
+        if (!ec && (bottom_up || p->max_degree <= LOW_DEGREE)) kc.threads = 512;
+        if (ec && !bottom_up && !p->mark_pred && p->edges >= (1ll << 23)) kc.threads = 256;
+    }
+    if (bottom_up) {
+        if (p->mark_pred && p->mask_snap_cap < p->mask_bytes) {
+            cudaFree(p->d_mask_snap);
+            p->d_mask_snap = nullptr;
+            p->mask_snap_cap = 0;
+            CUDA_TRY(cudaMalloc(&p->d_mask_snap, p->mask_bytes), "cudaMalloc visited-mask copy");
+            p->mask_snap_cap = p->mask_bytes;
         }
+        if ((rc = ensure_heavy_known(p))) return rc;
+        bp.mask_snap = p->d_mask_snap;
+        bp.heavy = p->d_heavy;
+        // the problem's row offsets, mask and keys carry the padding, and
+        // the expand-contract launch the stage buffers
+        kc.stage_bu = e->stage_bu && ec;
+        bp.stage_bu = kc.stage_bu ? 1 : 0;
+        bp.do_alpha = e->do_alpha;
+        bp.do_beta = e->do_beta;
+        if (!ec) bp.count_raw = 1;  // the edge frontiers decide the direction
     }
     if (bp.levels)
         CUDA_TRY(cudaMemsetAsync(bp.levels, 0, sizeof(LevelRecord) * LEVEL_LOG_CAP, s), "level log clear");
@@ -539,6 +554,30 @@ int set_persist_window(b40c_enactor *e, b40c_problem *p, cudaStream_t s, bool on
     return B40C_SUCCESS;
 }
 
+// The fused kernel's grid limit, asked for once per launch configuration.
+int fused_limit(b40c_enactor *e, const KernelConfig &kc, int *limit) {
+    const int key = (kc.threads << 2) | (kc.mark_pred ? 2 : 0) | (kc.stage_bu ? 1 : 0);
+    if (e->fused_key != key) {
+        CUDA_TRY(fused_grid_limit(kc, &e->fused_limit), "occupancy query");
+        e->fused_key = key;
+    }
+    *limit = e->fused_limit;
+    return B40C_SUCCESS;
+}
+
+// CTAs for a graph of `edges` entries: its levels' chains and barriers are
+// shorter on fewer CTAs until the largest level needs them all.  One per 8192
+// edges, at least 32, and half the limit (one per SM with 512 threads) below
+// 2^23 edges (at 2^24 half the limit is slower: two-phase on a directed R-MAT
+// scale 20 370 -> 403 us): R-MAT ef 16, contract-expand, scale 12 62.5 -> 52.7 us on 32,
+// scale 14 70 -> 60 us on 64, scale 16 69 -> 62 us and scale 18 115 -> 104 us on
+// 148 of 296; expand-contract 2 to 10% there.  Predecessor searches keep the
+// full grid (the CTAs' pace decides which parent is recorded).
+int small_graph_grid(long long edges, int limit) {
+    if (edges >= (1ll << 23)) return limit;
+    return int(std::max<long long>(std::min(32, limit), std::min<long long>(edges / 8192, std::max(1, limit / 2))));
+}
+
 // The launches of one search on stream s (init kernel, then the fused kernel
 // or the per-level graph), bracketed by the enactor's timing events.
 int launch_search(b40c_enactor *e, BfsParams &bp, const KernelConfig &kc, cudaStream_t s, int max_grid_size,
@@ -549,9 +588,10 @@ int launch_search(b40c_enactor *e, BfsParams &bp, const KernelConfig &kc, cudaSt
     if (variant == B40C_VARIANT_FUSED) {
         int limit = 0;
         if (low) limit = e->low_grid[low_degree_class(kc.low_degree)];
-        else CUDA_TRY(fused_grid_limit(kc, &limit), "occupancy query");
+        else if (int rc = fused_limit(e, kc, &limit)) return rc;
         int grid = max_grid_size > 0 ? std::min(max_grid_size, limit) : limit;
         if (low) grid -= grid % LF_TEAM;
+        else if (max_grid_size <= 0 && !kc.mark_pred) grid = std::min(grid, small_graph_grid(bp.edges, limit));
         e->busy_grid = 0;
         if (e->instrument) {
             if (e->busy_cap < grid) {
@@ -566,12 +606,14 @@ int launch_search(b40c_enactor *e, BfsParams &bp, const KernelConfig &kc, cudaSt
         }
         if (kc.strategy == B40C_CONTRACT_EXPAND || kc.strategy == B40C_HYBRID) bp.flat_max = e->flat_max;
         if (low) {
-            if (!e->d_starts)  // the two row-start queues, then the counts
-                CUDA_TRY(cudaMalloc(&e->d_starts, 2 * sizeof(int) * size_t(LF_STARTS) + LF_COUNTS * sizeof(uint2)),
-                         "cudaMalloc row-start queues");
-            LowDegreeParams lp{{e->d_starts, e->d_starts + LF_STARTS},
-                               reinterpret_cast<uint2 *>(e->d_starts + 2 * LF_STARTS),
-                               e->strategy, kc.low_degree};
+            // These searches have no chunks: the tables hold the row starts
+            // and the CTAs' counts instead.
+            static_assert(LF_COUNTS * sizeof(uint2) <= CHUNK_ENTRIES_MIN * sizeof(int4), "counts fit a chunk table");
+            const LowDegreeParams lp{{reinterpret_cast<int *>(e->d_wchunks[0]), reinterpret_cast<int *>(e->d_wchunks[1])},
+                                     unsigned(std::min<long long>(4ll * e->wchunk_cap, 1ll << 30)),
+                                     reinterpret_cast<uint2 *>(e->d_chunks[0]),
+                                     e->strategy,
+                                     kc.low_degree};
             CUDA_TRY(launch_low_degree(bp, lp, grid, s), "cooperative launch of the low-degree BFS kernel");
         } else if (e->narrow_team > 0) {
             // the launch's shared memory depends on all but the team: a new
@@ -1041,14 +1083,15 @@ extern "C" int b40c_enactor_create(int strategy, int instrument, int debug, b40c
     b40c_enactor *e = new (std::nothrow) b40c_enactor();
     if (!e) return set_error(B40C_ERR_MEMORY_ALLOCATION, "enactor allocation");
     e->strategy = strategy;
-    // Measured defaults: 512-thread CTAs (best on R-MAT scale 22 and on the
-    // lattices; the edge-frontier strategies' direction switch needs them).
+    // Measured defaults: expand-contract and contract-expand run 512-thread
+    // CTAs (best for both on R-MAT scale 22 and on the lattices), two-phase and
+    // the hybrid 256 (enqueue_search says where a search differs).
     // Expand-contract gathers lists of 128+ edges with warps, the others lists
     // of 64+, and every strategy switches direction with the published alpha =
     // 14, beta = 24 (Beamer, Asanovic and Patterson, SC 2012).
-    e->threads = 512;
     e->do_alpha = 14;
     e->do_beta = 24;
+    if (strategy == B40C_EXPAND_CONTRACT || strategy == B40C_CONTRACT_EXPAND) e->threads = 512;
     if (strategy == B40C_EXPAND_CONTRACT) e->warp_th = 128;
     e->instrument = instrument != 0;
     e->debug = debug != 0;
@@ -1056,8 +1099,10 @@ extern "C" int b40c_enactor_create(int strategy, int instrument, int debug, b40c
     if (!ce) ce = cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking);
     if (!ce) ce = cudaEventCreate(&e->ev0);
     if (!ce) ce = cudaEventCreate(&e->ev1);
+    if (!ce) ce = cudaEventCreateWithFlags(&e->dep, cudaEventDisableTiming);
     if (ce) {
         if (e->ev0) cudaEventDestroy(e->ev0);
+        if (e->ev1) cudaEventDestroy(e->ev1);
         if (e->own_stream) cudaStreamDestroy(e->own_stream);
         delete e;
         return cuda_fail(ce, "enactor creation");
@@ -1080,12 +1125,12 @@ extern "C" int b40c_enactor_destroy(b40c_enactor_t *e) {
     cudaFree(e->d_chunks[1]);
     cudaFree(e->d_wchunks[0]);
     cudaFree(e->d_wchunks[1]);
-    cudaFree(e->d_starts);
     cudaFree(e->d_levels);
     cudaFree(e->d_busy);
     if (e->h_ctr) cudaFreeHost(e->h_ctr);
     cudaEventDestroy(e->ev0);
     cudaEventDestroy(e->ev1);
+    cudaEventDestroy(e->dep);
     if (e->own_stream) cudaStreamDestroy(e->own_stream);
     delete e;
     return B40C_SUCCESS;
@@ -1125,11 +1170,8 @@ extern "C" int b40c_enact_search_async(b40c_enactor_t *e, b40c_problem_t *p, int
     // Order later problem-stream work (reset, extract) after the search.
     cudaStream_t ps = problem_stream(p), s = enactor_stream(e);
     if (ps != s) {
-        cudaEvent_t dep;
-        CUDA_TRY(cudaEventCreateWithFlags(&dep, cudaEventDisableTiming), "cudaEventCreate");
-        cudaEventRecord(dep, s);
-        cudaStreamWaitEvent(ps, dep, 0);
-        cudaEventDestroy(dep);
+        cudaEventRecord(e->dep, s);
+        cudaStreamWaitEvent(ps, e->dep, 0);
     }
     return B40C_SUCCESS;
 }
@@ -1178,7 +1220,10 @@ extern "C" int b40c_enactor_set_policy(b40c_enactor_t *e, int cta_threads, int w
         return set_error(B40C_ERR_INVALID_VALUE, "cta_threads must be 128, 256 or 512");
     if (warp_th < 0 || cta_th < 0 || cull_flags < -1 || cull_flags > 3)
         return set_error(B40C_ERR_INVALID_VALUE, "invalid policy field");
-    if (cta_threads) e->threads = cta_threads;
+    if (cta_threads) {
+        e->threads = cta_threads;
+        e->threads_user = true;
+    }
     if (warp_th) e->warp_th = warp_th;
     if (cta_th) e->cta_th = cta_th;
     if (cull_flags >= 0) e->cull_flags = unsigned(cull_flags);

@@ -3062,13 +3062,15 @@ static LevelFns pick_level(const KernelConfig &kc) {
     return kc.mark_pred ? level_fns_t<true>(kc.threads, kc.strategy) : level_fns_t<false>(kc.threads, kc.strategy);
 }
 
-static cudaError_t grid_for(const void *fn, int threads, size_t smem, int *grid) {
+// smem_max: the dynamic shared memory any launch of fn may ask for (opted in
+// once here, so that launches need not).
+static cudaError_t grid_for(const void *fn, int threads, size_t smem, size_t smem_max, int *grid) {
     int dev = 0, sms = 0, occ = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e) return e;
-    if ((e = allow_smem(fn, smem))) return e;
+    if ((e = allow_smem(fn, smem_max))) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem);
     if (e) return e;
     if (occ < 1) return cudaErrorInvalidConfiguration;
@@ -3084,7 +3086,9 @@ cudaError_t launch_search_init(const BfsParams &p, const KernelConfig &kc, cudaS
 }
 
 cudaError_t fused_grid_limit(const KernelConfig &kc, int *grid) {
-    return grid_for((const void *)pick_fused(kc), kc.threads, fused_smem_bytes(kc), grid);
+    KernelConfig staged = kc;
+    staged.stage_bu = true;
+    return grid_for((const void *)pick_fused(kc), kc.threads, fused_smem_bytes(kc), fused_smem_bytes(staged), grid);
 }
 
 cudaError_t level_grid_limit(const KernelConfig &kc, int *grid) {
@@ -3093,7 +3097,7 @@ cudaError_t level_grid_limit(const KernelConfig &kc, int *grid) {
         cudaError_t e = allow_smem((const void *)f.level_b, smem_bytes(kc));
         if (e) return e;
     }
-    return grid_for((const void *)f.level_a, kc.threads, smem_bytes(kc), grid);
+    return grid_for((const void *)f.level_a, kc.threads, smem_bytes(kc), smem_bytes(kc), grid);
 }
 
 cudaError_t launch_symmetry_hash(const int *row_offsets, const int *col, int nodes, long long edges,
@@ -3138,12 +3142,10 @@ cudaError_t launch_csr_check(const int *row_offsets, const int *col, int nodes, 
 
 cudaError_t launch_fused(const BfsParams &p, const KernelConfig &kc, int grid, cudaStream_t stream) {
     KernelFn fn = pick_fused(kc);
-    const size_t smem = fused_smem_bytes(kc);
-    cudaError_t e = allow_smem((const void *)fn, smem);
-    if (e) return e;
     BfsParams arg = p;
     void *args[] = {&arg};
-    return cudaLaunchCooperativeKernel((const void *)fn, dim3(grid), dim3(kc.threads), args, smem, stream);
+    return cudaLaunchCooperativeKernel((const void *)fn, dim3(grid), dim3(kc.threads), args, fused_smem_bytes(kc),
+                                       stream);
 }
 
 cudaError_t build_level_graph(BfsParams &p, const KernelConfig &kc, int grid, cudaGraphExec_t *exec,

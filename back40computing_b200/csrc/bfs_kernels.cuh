@@ -132,7 +132,8 @@ struct KernelConfig {
 
 // Enqueues the per-search initialisation (counters, source) on stream.
 cudaError_t launch_search_init(const BfsParams &p, const KernelConfig &kc, cudaStream_t stream);
-// Largest co-resident grid of the fused kernel (SMs x occupancy).
+// Largest co-resident grid of the fused kernel (SMs x occupancy); opts the
+// kernel in to its shared memory, so it comes before its first launch_fused.
 cudaError_t fused_grid_limit(const KernelConfig &kc, int *grid);
 // Grid of the per-level kernels (SMs x occupancy).
 cudaError_t level_grid_limit(const KernelConfig &kc, int *grid);
@@ -173,11 +174,13 @@ cudaError_t build_level_graph(BfsParams &p, const KernelConfig &kc, int grid,
 // Low-degree searches (low_degree.cu): depth labels, fused, no list of more
 // than LOW_DEGREE edges, nodes < LF_NODES.
 constexpr int LF_TEAM = 16;                  // CTAs of a cluster
-constexpr unsigned LF_STARTS = 1u << 20;     // entries of the row-start side queues
 constexpr unsigned LF_COUNTS = 2 * 512;      // entries of LowDegreeParams::counts
 constexpr long long LF_NODES = 1ll << 27;    // ids share a word with the list length
 struct LowDegreeParams {
-    int *starts[2];  // LF_STARTS row starts beside the first entries of queue[0] and queue[1]
+    // Row starts beside the first starts_cap entries of queue[0] and queue[1]
+    // (entries past them look theirs up).
+    int *starts[2];
+    unsigned starts_cap;
     uint2 *counts;   // LF_COUNTS: by level parity, what each CTA discovered (vertices, their edges)
     int strategy;    // whose statistics and level log the search reports
     int max_degree;

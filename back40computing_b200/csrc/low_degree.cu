@@ -339,11 +339,11 @@ __device__ __forceinline__ void grid_rounds(const BfsParams &p, const LowDegreeP
 #pragma unroll
         for (int u = 0; u < U; u++) {
             w[u] = pos[u] != ~0u ? (unsigned)ld_cg(q_in + pos[u]) : 0u;
-            col[u] = pos[u] < LF_STARTS ? ld_cg(s_in + pos[u]) : 0;
+            col[u] = pos[u] < a.starts_cap ? ld_cg(s_in + pos[u]) : 0;
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (pos[u] >= LF_STARTS && pos[u] != ~0u) col[u] = __ldg(p.row_offsets + (w[u] & ID_MASK));
+            if (pos[u] >= a.starts_cap && pos[u] != ~0u) col[u] = __ldg(p.row_offsets + (w[u] & ID_MASK));
             if (j < w[u] >> LEN_SHIFT) have |= 1u << u;
             col[u] += int(j);
         }
@@ -389,7 +389,7 @@ __device__ __forceinline__ bool grid_level(const BfsParams &p, const LowDegreePa
             const unsigned pos = base + k;
             if ((long long)pos < p.qcap) {
                 q_out[pos] = sm.stage[k].x;
-                if (pos < LF_STARTS) s_out[pos] = sm.stage[k].y;
+                if (pos < a.starts_cap) s_out[pos] = sm.stage[k].y;
             } else {
                 atomicOr(&p.ctr->error, ERR_OVERFLOW);
             }
@@ -459,7 +459,7 @@ __device__ __forceinline__ void cluster_levels(const BfsParams &p, const LowDegr
             }
             const unsigned w = (unsigned)ld_cg(q_in + pos);
             sm.region[0][s][k] =
-                make_int2(int(w), pos < LF_STARTS ? ld_cg(s_in + pos) : __ldg(p.row_offsets + (w & ID_MASK)));
+                make_int2(int(w), pos < a.starts_cap ? ld_cg(s_in + pos) : __ldg(p.row_offsets + (w & ID_MASK)));
         }
         if (threadIdx.x < 2) sm.found[threadIdx.x] = sm.edges[threadIdx.x] = 0u;
         cluster_sync_all();
@@ -522,7 +522,7 @@ __device__ __forceinline__ void cluster_levels(const BfsParams &p, const LowDegr
             const int2 e = sm.region[b ^ 1][s][k];
             const unsigned pos = before + k * TEAM + r;  // the sender's k * TEAM + r-th entry
             q[pos] = e.x;
-            st[pos] = e.y;
+            if (pos < a.starts_cap) st[pos] = e.y;
         }
     }
     if (threadIdx.x < 2) sm.found[threadIdx.x] = sm.edges[threadIdx.x] = 0u;

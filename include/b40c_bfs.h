@@ -147,7 +147,8 @@ int b40c_enactor_last_elapsed_ms(b40c_enactor_t *enactor, float *ms);
 int b40c_enactor_set_stream(b40c_enactor_t *enactor, void *stream);
 /* Tuning policy (the reference's compile-time KernelPolicy, kernel_policy.cuh:61-87,
  * WARP_GATHER_THRESHOLD / CTA_GATHER_THRESHOLD): cta_threads in {128,256,512}
- * (default 512);
+ * (default 512 for expand-contract and contract-expand, 256 for the others;
+ * unless set, a search takes 512 or 256 where that is faster for its graph);
  * lists of at least cta_gather_threshold edges (default 1024) are cut into
  * chunks of 16 * cta_threads edges, each gathered by a whole CTA; lists of at
  * least warp_gather_threshold edges (default 128 for expand-contract, 64 for
@@ -235,8 +236,11 @@ int b40c_enactor_set_bottom_up_staging(b40c_enactor_t *enactor, int enable);
  *    thread, short lists copied by their own thread, one queue reservation
  *    per CTA) instead of the tiled one (grid_frontier = 0: never;
  *    expand-contract and two-phase ignore it).
- * Both are off by default.  Results are the same either way.  No counterpart
- * in the reference. */
+ * Both are off by default.  Results are the same either way.  Depth-label
+ * searches of graphs without a list of more than 16 edges run a kernel of
+ * their own for every strategy and need neither (they ignore both, and the
+ * policy; it is used unless expand-contract's direction switch was set or
+ * max_grid_size is below 16).  No counterpart in the reference. */
 int b40c_enactor_set_narrow_levels(b40c_enactor_t *enactor, int team_ctas, int max_frontier,
                                    int grid_frontier);
 /* The cluster size narrow levels run on for depth-label searches with the
